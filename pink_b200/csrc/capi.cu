@@ -515,7 +515,7 @@ int train_chunk(pink_b200_ctx* c, const float* d_images, uint64_t m, uint32_t* l
         if (ev) CU_TRY(cudaEventRecord(ev[0], c->rot_stream));
         CU_TRY(cudaMemsetAsync(c->d_rmax + slot, 0, cnt * sizeof(uint32_t), c->rot_stream));
         LAUNCH_TRY(launch_rotate(g, d_images + s0 * isz, cnt, c->d_cs, c->d_sn,
-                                 c->d_base + slot * (g.q ? g.q : 1) * (size_t)g.P,
+                                 c->d_base + slot * (g.q ? g.q : 1) * (size_t)g.P, g.nd * g.nd,
                                  static_cast<uint8_t*>(c->d_b0) + row0 * g.Kp * esz,
                                  c->d_b1 ? static_cast<uint8_t*>(c->d_b1) + row0 * g.Kp * esz : nullptr,
                                  static_cast<uint8_t*>(c->d_bnorm) + row0 * (g.mode == kModeU16 ? 8 : 4),
@@ -572,7 +572,7 @@ static int train_chunk_shared(pink_b200_ctx* c, const float* d_images, uint64_t 
                 ev = &c->prof_rot_events[2 * c->prof_rot_used++];
             if (ev) CU_TRY(cudaEventRecord(ev[0], c->stream));
             LAUNCH_TRY(launch_rotate(g, d_images + (b * kRotBatch + lo) * isz, hi - lo, c->d_cs, c->d_sn,
-                                     c->d_base + (slot + lo) * nbase * (size_t)g.P,
+                                     c->d_base + (slot + lo) * nbase * (size_t)g.P, g.nd * g.nd,
                                      static_cast<uint8_t*>(c->d_b0) + row0 * g.Kp * esz,
                                      c->d_b1 ? static_cast<uint8_t*>(c->d_b1) + row0 * g.Kp * esz : nullptr,
                                      static_cast<uint8_t*>(c->d_bnorm) + row0 * (g.mode == kModeU16 ? 8 : 4),
@@ -1293,10 +1293,10 @@ static int map_chunk(pink_b200_ctx* c, const float* d_images, uint32_t m, float*
         int rc = ensure_filter_buffers(c, c->map_batch);
         if (rc) return rc;
         // the rotation kernel also writes the estimate's TF32 planes and norms of the transforms
-        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, c->d_b0, c->d_bf_hi,
+        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, g.nd * g.nd, c->d_b0, c->d_bf_hi,
                                  c->d_bf_norm, c->stream, nullptr, c->d_bf_lo));
     } else {
-        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, c->d_b0, c->d_b1, c->d_bnorm, c->stream));
+        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, g.nd * g.nd, c->d_b0, c->d_b1, c->d_bnorm, c->stream));
     }
     DistanceArgs da{};
     da.a0 = c->d_a0; da.a1 = c->d_a1; da.anorm = c->d_anorm; da.n = c->count;
@@ -1600,7 +1600,7 @@ int pink_b200_op_rotate(const pink_b200_config* cfg, const float* dev_images, ui
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     rc = stage_tables(g, &d_cs, &d_sn, st);
     if (rc) return rc;
-    cudaError_t e = launch_rotate(g, dev_images, n_img, d_cs, d_sn, dev_base, dev_b0, dev_b1, dev_bnorm, st);
+    cudaError_t e = launch_rotate(g, dev_images, n_img, d_cs, d_sn, dev_base, g.nd * g.nd, dev_b0, dev_b1, dev_bnorm, st);
     cudaStreamSynchronize(st);
     cudaFree(d_cs); cudaFree(d_sn);
     if (e != cudaSuccess) return fail(PINK_B200_ECUDA, std::string("rotate_kernel launch: ") + cudaGetErrorString(e));

@@ -59,15 +59,17 @@ struct BmuPair { unsigned long long code; unsigned long long neuron; };
 
 // ---- rotation set -----------------------------------------------------------
 // images: [n_img][C][id][id] float.  cs/sn: [q] cos/sin of t*2*pi/R (entry 0 unused).
-// base_out (nullable): [n_img][max(q,1)][C][nd][nd] float base rotations.
+// base_out (nullable): [n_img][max(q,1)][C] float base rotations, base_plane (>= nd*nd) floats from one nd x nd plane to the next;
+// required when the distance region of a base rotation does not fit shared memory.
 // b0/b1: operand planes [n_img*T][Kp] (u8: b0; u16: b0 = high byte, b1 = low
 // byte; f32: b0 as float, and -- when b1 is given -- b1 / b2 the two TF32 word
 // planes of the mapping estimate: value with its low 13 mantissa bits cleared,
 // and the rest).  bnorm: [n_img*T] sum of squares (u32 for u8, u64 for u16,
 // float for f32 with planes, else unused for f32).
-// rmax (nullable): [n_img] words zeroed by the caller; receives the bit pattern of max |pixel| over each image's base rotations.
+// rmax (nullable): [n_img] words zeroed by the caller; receives the bit pattern of an upper bound of
+// |pixel| over each image's base rotations.
 cudaError_t launch_rotate(const Geometry& g, const float* images, uint32_t n_img, const float* cs, const float* sn,
-                   float* base_out, void* b0, void* b1, void* bnorm, cudaStream_t st, uint32_t* rmax = nullptr,
+                   float* base_out, uint32_t base_plane, void* b0, void* b1, void* bnorm, cudaStream_t st, uint32_t* rmax = nullptr,
                    void* b2 = nullptr);
 
 // ---- SOM operand ------------------------------------------------------------

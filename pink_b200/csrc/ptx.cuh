@@ -135,6 +135,12 @@ __device__ __forceinline__ void bulk_wait_read_all()
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
+// The same for all but the most recent group.
+__device__ __forceinline__ void bulk_wait_read_one()
+{
+    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+}
+
 // Wait until all committed bulk stores are complete.
 __device__ __forceinline__ void bulk_wait_all()
 {
