@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 QDT = {0: np.float32, 1: np.uint8, 2: np.uint8}
 
 
-def _rotate(torch, capi, imgs, C_, idim, nd, ed, R, flip, mode):
+def _rotate(torch, capi, imgs, C_, idim, nd, ed, R, flip, mode, with_base=True):
     n_img = imgs.shape[0]
     T = R * (2 if flip else 1)
     q = max(R // 4, 1)
@@ -28,7 +28,7 @@ def _rotate(torch, capi, imgs, C_, idim, nd, ed, R, flip, mode):
     b0 = torch.zeros((n_img * T, Kp), dtype=tdt, device="cuda")
     b1 = torch.zeros((n_img * T, Kp), dtype=tdt, device="cuda") if mode == 1 else None
     bnorm = torch.zeros(n_img * T, dtype=torch.int64 if mode == 1 else torch.int32, device="cuda")
-    capi.check(capi.lib.pink_b200_op_rotate(C.byref(cfg), ptr(d_img), n_img, ptr(base), ptr(b0), ptr(b1), ptr(bnorm), None))
+    capi.check(capi.lib.pink_b200_op_rotate(C.byref(cfg), ptr(d_img), n_img, ptr(base) if with_base else None, ptr(b0), ptr(b1), ptr(bnorm), None))
     torch.cuda.synchronize()
     return base.cpu().numpy(), b0.cpu().numpy(), None if b1 is None else b1.cpu().numpy(), bnorm.cpu().numpy(), K, Kp
 
@@ -67,6 +67,46 @@ def test_rotation_set_and_operand(cuda, case, mode):
             assert np.array_equal(b1[rows, :K], (want & 255).astype(np.uint8))
             assert np.array_equal(bnorm[rows].astype(np.uint64), (want.astype(np.uint64) ** 2).sum(1))
         assert not b0[rows, K:].any(), "operand padding must stay zero"
+
+
+ROT_LAYOUTS = [
+    # C, id, nd, ed, flip: region rows of a multiple of 32 bytes, off-centre regions, one instead of two sets of operand
+    # rows, a float plane too large to stage, a region or an image too large to stage, neurons beyond the image
+    (1, 70, 50, 32, True), (1, 70, 49, 32, True), (1, 70, 48, 33, False), (1, 160, 113, 110, True), (1, 130, 183, 91, True),
+    (1, 300, 200, 180, True), (1, 24, 190, 181, True), (3, 90, 64, 47, True), (1, 4, 3, 2, True),
+]
+
+
+@pytest.mark.parametrize("case", ROT_LAYOUTS)
+@pytest.mark.parametrize("mode", [2, 1, 0])
+def test_rotation_layouts(cuda, case, mode):
+    """The layouts the rotation kernel chooses between, with and without base rotations to store."""
+    import pink_b200.capi as capi
+    C_, idim, nd, ed, flip = case
+    if mode == 1 and C_ * ed * ed > 16512:
+        pytest.skip("uint16 region limit")
+    R, n_img = 12, 2
+    rng = np.random.default_rng(nd * 1000 + ed)
+    imgs = rng.random((n_img, C_, idim, idim), dtype=np.float32)
+    base, b0, b1, bnorm, K, Kp = _rotate(cuda, capi, imgs, C_, idim, nd, ed, R, flip, mode)
+    got = [(b0, b1, bnorm)]
+    if nd <= 200:
+        got.append(_rotate(cuda, capi, imgs, C_, idim, nd, ed, R, flip, mode, with_base=False)[1:4])
+    T = R * (2 if flip else 1)
+    for i in range(n_img):
+        rot = O.rotation_set(imgs[i], nd, R, flip)
+        assert np.array_equal(base[i].view(np.uint32), rot[:R // 4].view(np.uint32))
+        want = O.crop_quantize(rot, ed, mode)
+        rows = slice(i * T, (i + 1) * T)
+        for b0, b1, bnorm in got:
+            if mode == 0:
+                assert np.array_equal(b0[rows, :K].view(np.uint32), want.view(np.uint32))
+            else:
+                value = b0[rows, :K].astype(np.uint16) if mode == 2 else b0[rows, :K].astype(np.uint16) << 8 | b1[rows, :K]
+                assert np.array_equal(value, want)
+                assert np.array_equal(bnorm[rows].view(np.uint64 if mode == 1 else np.uint32).astype(np.uint64),
+                                      (want.astype(np.uint64) ** 2).sum(1))
+            assert not b0[rows, K:].any()
 
 
 def _distance(torch, capi, a, b, mode, n_img=1, want_matrix=True):
