@@ -388,6 +388,8 @@ int train_step(pink_b200_ctx* c, size_t slot_img, uint32_t* bmu_slot)
     // Fused form: the update kernel reduces the keys (or the exchanged records) and derives its
     // work list itself; otherwise a reduction and a compaction kernel run in between.
     const bool fused = c->fuse_update;
+    ba.anorm = c->d_anorm;
+    ba.anorm_bytes = fused || g.mode == kModeF32 ? 0u : (g.mode == kModeU16 ? 8u : 4u);
     const bool multi = c->cfg.world_size > 1;
     const bool peer = multi && fused && c->xchg_on;
     if (peer) {

@@ -159,6 +159,7 @@ struct BmuArgs
     uint32_t neuron_stride;           // local neuron j is global neuron first_neuron + j * neuron_stride
     BmuPair* pairs; uint32_t rank, world;                        // per-rank records (world entries)
     FactorSource factors;             // update factors of (best matching unit, neuron)
+    void* anorm; uint32_t anorm_bytes;   // phase 2: sums of squares (4 or 8 bytes each) the unfused update adds up anew; 0: none
     UpdateItem* items; uint32_t* n_items;   // out: neurons with a non-zero factor, ascending, and their number
     uint32_t* counts;                 // [N_global] BMU hit counters (incremented by the owner)
     uint32_t* bmu_log;                // nullable: receives the global BMU index of this step
@@ -183,7 +184,7 @@ struct UpdateArgs
     float* som;                       // [n][Pp]
     const float* base;                // [max(q,1)][C][nd][nd] base rotations of the current image
     const UpdateItem* items; const uint32_t* n_items;   // work list from launch_bmu
-    uint32_t n;                       // local neurons (upper bound of the work list)
+    uint32_t n, first_item;           // local neurons (upper bound of the work list); list entry `items` points at
     void* a0; void* a1; void* anorm;  // SOM operand rows to refresh
     // Fused form only (both nullable together): per-neuron {min |w|, max |w|} as float bit patterns,
     // kept up to date by the kernel, and the bit pattern of max |r| over the current image's base
@@ -208,7 +209,8 @@ __host__ __device__ inline bool cannot_change(float f, uint32_t wmin_bits, uint3
     return false;
 #endif
 }
-// Unfused form: one block per neuron works through the list launch_bmu (phase 2) wrote.
+// Unfused form: blocks work through the list launch_bmu (phase 2) wrote, strip by strip; the listed neurons' sums of
+// squares must be zero (BmuArgs::anorm).
 cudaError_t launch_update(const Geometry& g, const UpdateArgs& a, cudaStream_t st, int* status);
 // Fused form, a persistent pipelined kernel: it reduces the keys (world == 1) or the exchanged
 // per-rank records (world > 1, after launch_bmu phase 1 and the exchange) to the best matching unit,

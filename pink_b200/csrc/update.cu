@@ -14,7 +14,7 @@
 // quantised distance operand row and its sum of squares.  The difference, the
 // product and the final subtraction are rounded separately (never contracted to
 // FMA), as in the reference's CPU loop (src/SelfOrganizingMapLib/Trainer.h:167-179).
-// bmu_kernel, worklist_kernel and update_kernel (one block per listed neuron)
+// bmu_kernel, worklist_kernel and update_kernel (a block per strip of a listed neuron)
 // are the same steps as separate kernels, for neurons too large for the
 // pipelined kernel's shared-memory stages.
 #include "kernels.cuh"
@@ -89,6 +89,8 @@ worklist_kernel(BmuArgs a)
     if (i < a.n) {
         a.keys[i] = kKeyEmpty;                          // re-arm every key for the next image's distance kernel
         if (f != 0.0f) {
+            if (a.anorm_bytes == 4) static_cast<uint32_t*>(a.anorm)[i] = 0u;
+            else if (a.anorm_bytes == 8) static_cast<unsigned long long*>(a.anorm)[i] = 0ull;
             a.items[slot] = make_item(a, i, key, f);
         }
     }
@@ -100,146 +102,85 @@ worklist_kernel(BmuArgs a)
 
 constexpr int kUpdThreads = 256;
 constexpr int kUpdWarps = kUpdThreads / 32;
-constexpr int kRowBatch = 12;         // neuron rows a thread keeps in flight (one float each)
+constexpr int kUpdRows = 8;           // rows a thread keeps in flight (one float each, four rows apart)
+constexpr uint32_t kStripRows = 4 * kUpdRows;
 
 // v / d for v * d < 2^32 with magic = floor(2^32 / d) + 1 (ranges checked on the host).
 // magic == 0 encodes the divisor 1.
 __device__ __forceinline__ uint32_t fast_div(uint32_t v, uint32_t magic) { return magic ? __umulhi(v, magic) : v; }
 inline uint32_t div_magic(uint32_t d) { return d == 1 ? 0u : (uint32_t)((1ull << 32) / d) + 1; }
 
-// Per neuron row (over all channels): where the row starts in the base
-// rotation under the neuron's best transform, and where it lands in the
-// distance operand (negative when the row lies outside the distance region).
-struct RowInfo { int32_t src; int32_t kk; uint32_t span; };   // span: region columns [low 16 bits, high 16 bits) of the row
-
-// One block per neuron of the shard.  The block looks up the best matching
-// unit and its own update factor, leaves at once when the factor is zero, and
-// otherwise walks the neuron in tasks of kRowBatch rows x 32 columns: a thread
-// owns one column of the task, so its global address, its source position in
-// the base rotation and its operand position advance by per-row constants
-// taken from a small shared table, and kRowBatch loads are in flight per
-// thread before anything depends on them.
+// One block per strip of kStripRows rows of a listed neuron's channel plane (x: channel and strip, y: work list entry).
+// The kernel moves 12 bytes per pixel and computes next to nothing, so what counts is how many loads are in flight on
+// all SMs: with one block per neuron a map of 100 neurons left a third of the SMs idle and the others with 134 KB to
+// walk by eight warps; strips of 32 rows give every SM several blocks.  Per
+// image: 72.2 -> 15.4 us (100 neurons of 183 x 183), 12.1 -> 4.4 us (63 of 71 x 71), 7.7 -> 3.2 us (64 of 45 x 45).  A warp's load covers 4 rows x 8 columns: the base
+// rotation is read through the quarter-turn permutation, and a tile of that shape touches whole 16- or 32-byte
+// runs either way round (a row of 32 pixels would touch 32 lines for the odd quarter turns).
+// The strips of a neuron add their sums of squares into anorm, which worklist_kernel has zeroed.
 template <int MODE>
-__global__ void __launch_bounds__(kUpdThreads, 4)
-update_kernel(Geometry g, UpdateArgs a, uint32_t stage_base, uint32_t magic_nd, uint32_t magic_blocks)
+__global__ void __launch_bounds__(kUpdThreads)
+update_kernel(const __grid_constant__ Geometry g, const __grid_constant__ UpdateArgs a, uint32_t strips)
 {
-    extern __shared__ __align__(16) uint8_t dyn[];
-    const uint32_t rows = g.C * g.nd;
-    RowInfo* rowinfo = reinterpret_cast<RowInfo*>(dyn);                                  // [rows]
-    uint8_t* crop_s = dyn + (((size_t)rows * sizeof(RowInfo) + 15) & ~size_t(15));       // operand row(s) being rebuilt
-    const size_t crop_bytes = MODE == kModeF32 ? (size_t)g.Kp * 4 : (MODE == kModeU16 ? (size_t)g.Kp * 2 : g.Kp);
-    float* base_s = reinterpret_cast<float*>(crop_s + ((crop_bytes + 15) & ~size_t(15))); // [P] base rotation
-    __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long red[kUpdWarps];
-
-    __shared__ UpdateItem item_s;
-    __shared__ uint32_t live_s;
-    if (threadIdx.x == 0) {
-        live_s = blockIdx.x < *a.n_items;
-        item_s = a.items[blockIdx.x];     // entries beyond n_items are stale but in bounds
-        mbar_init(&bar, 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    if (!live_s) return;                  // fewer neurons to update than blocks
-    const UpdateItem it = item_s;
-    const uint32_t n = it.n, tq = it.tq;
-    const float f = it.f;
-    const int32_t ax = it.ax, ay = it.ay, a0 = it.a0;
-    const float* bsrc = a.base + (size_t)tq * g.P;
-    if (stage_base && threadIdx.x == 0) {
-        // one bulk asynchronous copy (TMA) of the whole base rotation into shared memory
-        mbar_expect_tx(&bar, g.P * 4);
-        bulk_load(base_s, bsrc, g.P * 4, &bar);
-    }
-    const uint32_t P1 = g.nd * g.nd, K1 = g.ed * g.ed;
-    for (uint32_t rr = threadIdx.x; rr < rows; rr += kUpdThreads) {
-        const uint32_t c = fast_div(rr, magic_nd), x = rr - c * g.nd;
-        const uint32_t ci = x - g.off;                                   // unsigned wrap rejects x < off
-        rowinfo[rr].src = (int32_t)(c * P1) + ax * (int32_t)x + a0;
-        rowinfo[rr].kk = ci < g.ed ? (int32_t)(c * K1 + ci * g.ed) : -1;
-        uint32_t span = g.ed << 16;
-        if (g.circle && ci < g.ed) { const ushort2 r = g.circle[ci]; span = (uint32_t)r.x | ((uint32_t)r.y << 16); }
-        rowinfo[rr].span = span;
-    }
-    __syncthreads();
-
-    float* w = a.som + (size_t)n * g.Pp;
+    if (a.first_item + blockIdx.y >= *a.n_items) return;                // fewer neurons to update than the shard has
+    const UpdateItem it = a.items[blockIdx.y];
+    const uint32_t c = blockIdx.x / strips, xs = (blockIdx.x - c * strips) * kStripRows;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t blocks_per_col = (rows + kRowBatch - 1) / kRowBatch;
-    const uint32_t ntask = ((g.nd + 31) / 32) * blocks_per_col;
+    const uint32_t nd = g.nd, ed = g.ed, P1 = nd * nd, K1 = ed * ed;
+    const float* __restrict__ base = a.base + (size_t)it.tq * g.P + (size_t)c * P1;
+    float* w = a.som + (size_t)it.n * g.Pp + (size_t)c * P1;
+    uint8_t* row0 = static_cast<uint8_t*>(a.a0) + ((size_t)it.n * g.Kp + (size_t)c * K1) * (MODE == kModeF32 ? 4 : 1);
+    uint8_t* row1 = MODE == kModeU16 ? static_cast<uint8_t*>(a.a1) + (size_t)it.n * g.Kp + (size_t)c * K1 : nullptr;
+    const uint32_t x0 = xs + (lane >> 3);
     unsigned long long acc = 0;
-    bool staged = false;
-    for (uint32_t task = warp; task < ntask; task += kUpdWarps) {
-        const uint32_t col = fast_div(task, magic_blocks), row0 = (task - col * blocks_per_col) * kRowBatch;
-        const uint32_t y = col * 32 + lane;
-        const bool valid = y < g.nd;
-        const uint32_t cj = y - g.off;                                   // unsigned wrap rejects y < off
-        const bool in_col = cj < g.ed;
-        const int32_t ayy = ay * (int32_t)y;
-        float* p0 = w + (size_t)row0 * g.nd + y;
-        float v[kRowBatch];
+    for (uint32_t yt = warp; yt * 8 < nd; yt += kUpdWarps) {
+        const uint32_t y = yt * 8 + (lane & 7);
+        if (y >= nd) continue;
+        const int32_t src = it.a0 + it.ay * (int32_t)y + it.ax * (int32_t)x0;
+        float v[kUpdRows], r[kUpdRows];
 #pragma unroll
-        for (int u = 0; u < kRowBatch; ++u) {
-            v[u] = 0.0f;
-            if (valid && row0 + u < rows) v[u] = __ldcs(p0 + (size_t)u * g.nd);
+        for (int u = 0; u < kUpdRows; ++u) {
+            const bool ok = x0 + 4 * u < nd;
+            v[u] = ok ? __ldcs(w + (x0 + 4 * u) * nd + y) : 0.0f;
+            r[u] = ok ? __ldg(base + src + 4 * u * it.ax) : 0.0f;
         }
-        if (stage_base && !staged) {
-            if (!mbar_wait(&bar, 0)) return;      // bounded; cannot expire unless the copy faulted
-            bsrc = base_s;
-            staged = true;
-        }
+        const uint32_t cj = y - g.off;                   // unsigned wrap rejects y < off
 #pragma unroll
-        for (int u = 0; u < kRowBatch; ++u) {
-            if (valid && row0 + u < rows) {
-                const RowInfo ri = rowinfo[row0 + u];
-                const float rv = bsrc[ri.src + ayy];
-                const float nv = __fsub_rn(v[u], __fmul_rn(__fsub_rn(v[u], rv), f));
-                __stcs(p0 + (size_t)u * g.nd, nv);
-                if (in_col && ri.kk >= 0) {
-                    const uint32_t kk = (uint32_t)ri.kk + cj;
-                    const float ov = (cj >= (ri.span & 0xFFFFu) && cj < (ri.span >> 16)) ? nv : 0.0f;   // zero outside a circular region
+        for (int u = 0; u < kUpdRows; ++u) {
+            const uint32_t x = x0 + 4 * u, ci = x - g.off;
+            if (x < nd) {
+                const float nv = __fsub_rn(v[u], __fmul_rn(__fsub_rn(v[u], r[u]), it.f));
+                __stcs(w + x * nd + y, nv);
+                if (ci < ed && cj < ed && in_region(g, ci, cj)) {     // outside a circular region: stays zero
+                    const uint32_t kk = ci * ed + cj;
                     if (MODE == kModeU8) {
-                        const uint32_t qv = quant_u8(ov);
-                        crop_s[kk] = (uint8_t)qv;
+                        const uint32_t qv = quant_u8(nv);
+                        row0[kk] = (uint8_t)qv;
                         acc += qv * qv;
                     } else if (MODE == kModeU16) {
-                        const uint32_t qv = quant_u16(ov);
-                        crop_s[kk] = (uint8_t)(qv >> 8);
-                        crop_s[g.Kp + kk] = (uint8_t)(qv & 255);
+                        const uint32_t qv = quant_u16(nv);
+                        row0[kk] = (uint8_t)(qv >> 8);
+                        row1[kk] = (uint8_t)(qv & 255);
                         acc += (unsigned long long)qv * qv;
                     } else {
-                        reinterpret_cast<float*>(crop_s)[kk] = ov;
+                        reinterpret_cast<float*>(row0)[kk] = nv;
                     }
                 }
             }
         }
     }
-    __syncthreads();
-
-    // Operand row(s) back to global memory, 16 bytes per store; the padding
-    // beyond K stays as allocated (zero).
-    const uint32_t row_bytes = MODE == kModeF32 ? g.K * 4 : g.K;
-    const uint32_t stride_bytes = MODE == kModeF32 ? g.Kp * 4 : g.Kp;
-    const uint32_t planes = MODE == kModeU16 ? 2 : 1;
-    for (uint32_t pl = 0; pl < planes; ++pl) {
-        uint8_t* dst = static_cast<uint8_t*>(pl ? a.a1 : a.a0) + (size_t)n * stride_bytes;
-        const uint8_t* src = crop_s + (size_t)pl * g.Kp;
-        const uint32_t vecs = row_bytes / 16;
-        for (uint32_t i = threadIdx.x; i < vecs; i += blockDim.x)
-            reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
-        for (uint32_t i = vecs * 16 + threadIdx.x; i < row_bytes; i += blockDim.x) dst[i] = src[i];
-    }
     if (MODE != kModeF32) {
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         if (lane == 0) red[warp] = acc;
         __syncthreads();
         if (threadIdx.x == 0) {
             unsigned long long s = 0;
-            for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += red[i];
-            if (MODE == kModeU8) static_cast<uint32_t*>(a.anorm)[n] = (uint32_t)s;
-            else static_cast<unsigned long long*>(a.anorm)[n] = s;
+            for (int i = 0; i < kUpdWarps; ++i) s += red[i];
+            if (s != 0) {
+                if (MODE == kModeU8) atomicAdd(static_cast<uint32_t*>(a.anorm) + it.n, (uint32_t)s);
+                else atomicAdd(static_cast<unsigned long long*>(a.anorm) + it.n, s);
+            }
         }
     }
 }
@@ -769,28 +710,16 @@ __global__ void map_finalize_kernel(unsigned long long* __restrict__ keys, size_
 template <int MODE>
 cudaError_t update_classic(const Geometry& g, const UpdateArgs& a, cudaStream_t st)
 {
-    if ((uint64_t)g.P * g.nd >= (1ull << 32)) return cudaErrorInvalidValue;   // multiply-high division range
-    const size_t crop = MODE == kModeF32 ? (size_t)g.Kp * 4 : (MODE == kModeU16 ? (size_t)g.Kp * 2 : g.Kp);
-    const size_t rows = (size_t)g.C * g.nd;
-    const size_t fixed = ((rows * sizeof(RowInfo) + 15) & ~size_t(15)) + ((crop + 15) & ~size_t(15));
-    const size_t staged = fixed + (size_t)g.P * 4;
-    // The bulk copy needs a size that is a multiple of 16 bytes; otherwise (and
-    // when a base rotation does not fit) the base is read through the cache.
-    const uint32_t stage_base = staged <= 200 * 1024 && (g.P & 3) == 0;
-    const size_t smem = stage_base ? staged : fixed;
-    // Dynamic shared memory above 48 KB is an opt-in, per-device function attribute.
-    static thread_local int attr_dev = -1;
-    static thread_local size_t attr_bytes = 0;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (smem > 48 * 1024 && (dev != attr_dev || smem > attr_bytes)) {
-        cudaError_t e = cudaFuncSetAttribute(update_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr_dev = dev;
-        attr_bytes = smem;
+    const uint64_t strips = (g.nd + kStripRows - 1) / kStripRows, blocks = strips * g.C;
+    // (the rotation kernel sets the same limit for one channel)
+    if ((uint64_t)g.P * g.nd >= (1ull << 32) || blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+    // (a grid is at most 65535 high: longer lists go in several launches)
+    for (uint32_t n0 = 0; n0 < a.n; n0 += 65535u) {
+        UpdateArgs part = a;
+        part.items = a.items + n0;
+        part.first_item = n0;
+        update_kernel<MODE><<<dim3((unsigned)blocks, std::min(a.n - n0, 65535u)), kUpdThreads, 0, st>>>(g, part, (uint32_t)strips);
     }
-    const uint32_t blocks_per_col = (uint32_t)((rows + kRowBatch - 1) / kRowBatch);
-    update_kernel<MODE><<<a.n, kUpdThreads, smem, st>>>(g, a, stage_base, div_magic(g.nd), div_magic(blocks_per_col));
     return cudaGetLastError();
 }
 

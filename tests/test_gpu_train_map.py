@@ -98,6 +98,37 @@ def test_step_kernels_agree(cuda, case, mode):
         assert out[0][4][1] < read_s and out[0][4][0] < read_s
 
 
+SPLIT_CASES = [
+    # C, id, nd, ed, shape: strips of 32 rows and tiles of 8 columns -- below, at and above one strip, odd rows,
+    # several channels, a circular region, and neurons too large for the kernels that stage whole planes
+    (1, 40, 31, 31, 0), (1, 40, 32, 23, 0), (1, 44, 33, 20, 0), (3, 50, 35, 33, 0), (2, 50, 40, 17, 1), (1, 90, 121, 90, 0),
+    (1, 130, 183, 91, 0), (2, 100, 117, 65, 1),
+]
+
+
+@pytest.mark.parametrize("case", SPLIT_CASES)
+@pytest.mark.parametrize("mode", [2, 1])
+def test_split_update_bit_exact(cuda, case, mode):
+    """The reduction / work list / update kernels of option step_kernel = 2: map, units and (through the next step's
+    distances) operand rows and norms equal the oracle's bit for bit."""
+    import pink_b200.capi as capi
+    C_, idim, nd, ed, shape = case
+    N, R, n = 20, 8, 4
+    rng = np.random.default_rng(nd * 100 + ed + mode)
+    som0 = rng.random((N, C_, nd, nd), dtype=np.float32)
+    imgs = blob_images(n, idim, C_, seed=nd).reshape(n, C_, idim, idim)
+    F = O.update_factors(0, 5, 4, O.FUNC_GAUSSIAN, 1.1, 0.2)
+    want = som0.copy()
+    want_bmu = [O.train_step(want, im, F, ed, R, True, mode, shape=shape)[2] for im in imgs]
+    cfg = make_config(capi, N, C_, idim, nd, ed, R, True, mode)
+    cfg.ed_shape = capi.CIRCULAR if shape else capi.QUADRATIC
+    with Context(capi, cfg, {"step_kernel": 2}) as ctx:
+        ctx.set_som(som0)
+        ctx.set_factors(F)
+        assert list(ctx.train(imgs)) == want_bmu
+        assert np.array_equal(ctx.get_som(som0).view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("case", TRAIN_CASES[:5])
 def test_train_float_mode(cuda, case):
     """float32: one teacher-forced step at a time; the SOM must match the oracle bit for bit whenever
