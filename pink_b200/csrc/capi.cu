@@ -105,7 +105,7 @@ int make_geometry(const pink_b200_config& c, Geometry* g)
     g->off = static_cast<uint32_t>((g->nd - g->ed) * 0.5);
     const uint64_t P = (uint64_t)g->C * g->nd * g->nd, K = (uint64_t)g->C * g->ed * g->ed;
     if (P > (1u << 30)) return fail(PINK_B200_EINVAL, "neuron size too large");
-    g->P = (uint32_t)P; g->Pp = round_up(g->P, 4);
+    g->P = (uint32_t)P; g->Pc = round_up(g->nd * g->nd, 4); g->Pp = g->C * g->Pc;
     g->K = (uint32_t)K;
     g->mode = (int)c.dist_type;
     g->circle = nullptr;             // a context with a circular region uploads the table and sets this
@@ -277,7 +277,7 @@ int ensure_transform_buffers(pink_b200_ctx* c, size_t imgs, size_t base_needed)
     }
     if (c->base_imgs < base_needed) {
         free_dev(c->d_base);
-        CU_TRY(cudaMalloc(&c->d_base, base_needed * (g.q ? g.q : 1) * (size_t)g.P * sizeof(float)));
+        CU_TRY(cudaMalloc(&c->d_base, base_needed * (g.q ? g.q : 1) * (size_t)g.Pp * sizeof(float)));
         c->base_imgs = base_needed;
     }
     const size_t key_imgs_needed = imgs;
@@ -437,7 +437,7 @@ int train_step(pink_b200_ctx* c, size_t slot_img, uint32_t* bmu_slot)
     }
     UpdateArgs ua{};
     ua.som = c->d_som;
-    ua.base = c->d_base + slot_img * (g.q ? g.q : 1) * (size_t)g.P;
+    ua.base = c->d_base + slot_img * (g.q ? g.q : 1) * (size_t)g.Pp;
     ua.items = c->d_items; ua.n_items = c->d_nitems; ua.n = c->count;
     ua.a0 = c->d_a0; ua.a1 = c->d_a1; ua.anorm = c->d_anorm;
     ua.wrange = fused ? c->d_wrange : nullptr;
@@ -462,7 +462,7 @@ int train_steps_batch(pink_b200_ctx* c, size_t slot_img, uint32_t cnt, uint32_t*
     a.b_row0 = (uint32_t)(slot_img * g.T);
     a.keys = c->d_keys;
     a.som = c->d_som;
-    a.base = c->d_base + slot_img * (g.q ? g.q : 1) * (size_t)g.P;
+    a.base = c->d_base + slot_img * (g.q ? g.q : 1) * (size_t)g.Pp;
     a.wrange = c->d_wrange;
     a.rmax = c->d_wrange ? c->d_rmax + slot_img : nullptr;
     a.factors = c->factor_source;
@@ -517,7 +517,7 @@ int train_chunk(pink_b200_ctx* c, const float* d_images, uint64_t m, uint32_t* l
         if (ev) CU_TRY(cudaEventRecord(ev[0], c->rot_stream));
         CU_TRY(cudaMemsetAsync(c->d_rmax + slot, 0, cnt * sizeof(uint32_t), c->rot_stream));
         LAUNCH_TRY(launch_rotate(g, d_images + s0 * isz, cnt, c->d_cs, c->d_sn,
-                                 c->d_base + slot * (g.q ? g.q : 1) * (size_t)g.P, g.nd * g.nd,
+                                 c->d_base + slot * (g.q ? g.q : 1) * (size_t)g.Pp, g.Pc,
                                  static_cast<uint8_t*>(c->d_b0) + row0 * g.Kp * esz,
                                  c->d_b1 ? static_cast<uint8_t*>(c->d_b1) + row0 * g.Kp * esz : nullptr,
                                  static_cast<uint8_t*>(c->d_bnorm) + row0 * (g.mode == kModeU16 ? 8 : 4),
@@ -554,7 +554,7 @@ static int train_chunk_shared(pink_b200_ctx* c, const float* d_images, uint64_t 
     // the ranks sharing with this one: [g0, g0 + G), this rank the gr-th of them
     const uint32_t g0 = rank / c->share_group * c->share_group, G = std::min(c->share_group, W - g0), gr = rank - g0;
     const size_t esz = g.mode == kModeF32 ? 4 : 1, isz = c->image_size(), nbase = g.q ? g.q : 1;
-    const size_t base_img = nbase * (size_t)g.P * sizeof(float), op_img = (size_t)g.T * g.Kp * esz;
+    const size_t base_img = nbase * (size_t)g.Pp * sizeof(float), op_img = (size_t)g.T * g.Kp * esz;
     const size_t norm_img = (size_t)g.T * (g.mode == kModeU16 ? 8 : 4);
     if (ready) CU_TRY(cudaStreamWaitEvent(c->stream, ready, 0));
     const uint64_t batches = (m + kRotBatch - 1) / kRotBatch;
@@ -574,7 +574,7 @@ static int train_chunk_shared(pink_b200_ctx* c, const float* d_images, uint64_t 
                 ev = &c->prof_rot_events[2 * c->prof_rot_used++];
             if (ev) CU_TRY(cudaEventRecord(ev[0], c->stream));
             LAUNCH_TRY(launch_rotate(g, d_images + (b * kRotBatch + lo) * isz, hi - lo, c->d_cs, c->d_sn,
-                                     c->d_base + (slot + lo) * nbase * (size_t)g.P, g.nd * g.nd,
+                                     c->d_base + (slot + lo) * nbase * (size_t)g.Pp, g.Pc,
                                      static_cast<uint8_t*>(c->d_b0) + row0 * g.Kp * esz,
                                      c->d_b1 ? static_cast<uint8_t*>(c->d_b1) + row0 * g.Kp * esz : nullptr,
                                      static_cast<uint8_t*>(c->d_bnorm) + row0 * (g.mode == kModeU16 ? 8 : 4),
@@ -805,6 +805,28 @@ int setup_peer_exchange(pink_b200_ctx* c)
             if (!c->bcast_done[i]) CU_TRY(cudaEventCreateWithFlags(&c->bcast_done[i], cudaEventDisableTiming));
     }
     return PINK_B200_OK;
+}
+
+// This shard's neurons between a whole map in host memory (dense) and the device (padded channel planes).
+cudaError_t copy_som(pink_b200_ctx* c, float* host_som, cudaMemcpyKind kind)
+{
+    const Geometry& g = c->g;
+    const bool up = kind == cudaMemcpyHostToDevice;
+    float* host = host_som + (size_t)c->first * g.P;
+    const size_t host_pitch = (size_t)c->stride * g.P * sizeof(float), dev_pitch = (size_t)g.Pp * sizeof(float);
+    if (g.C == 1 || g.P == g.Pp)
+        return up ? cudaMemcpy2DAsync(c->d_som, dev_pitch, host, host_pitch, (size_t)g.P * sizeof(float), c->count, kind, c->stream)
+                  : cudaMemcpy2DAsync(host, host_pitch, c->d_som, dev_pitch, (size_t)g.P * sizeof(float), c->count, kind, c->stream);
+    // rows are channel planes, slices neurons
+    const size_t plane = (size_t)g.nd * g.nd * sizeof(float), padded = (size_t)g.Pc * sizeof(float);
+    const cudaPitchedPtr h = make_cudaPitchedPtr(host, plane, plane, (size_t)g.C * c->stride);
+    const cudaPitchedPtr d = make_cudaPitchedPtr(c->d_som, padded, padded, g.C);
+    cudaMemcpy3DParms p = {};
+    p.srcPtr = up ? h : d;
+    p.dstPtr = up ? d : h;
+    p.extent = make_cudaExtent(plane, g.C, c->count);
+    p.kind = kind;
+    return cudaMemcpy3DAsync(&p, c->stream);
 }
 
 int train_prepare(pink_b200_ctx* c, uint64_t n)
@@ -1112,9 +1134,7 @@ int pink_b200_set_som(pink_b200_ctx* c, const float* host_som)
     // Stream-ordered copy: a blocking cudaMemcpy from pageable memory may return
     // while its DMA is still in flight on the legacy stream, which the
     // context's non-blocking stream does not wait for.
-    CU_TRY(cudaMemcpy2DAsync(c->d_som, (size_t)g.Pp * sizeof(float), host_som + (size_t)c->first * g.P,
-                             (size_t)c->stride * g.P * sizeof(float), (size_t)g.P * sizeof(float), c->count,
-                             cudaMemcpyHostToDevice, c->stream));
+    CU_TRY(copy_som(c, const_cast<float*>(host_som), cudaMemcpyHostToDevice));
     if ((c->fuse_update || c->plan_ok) && !c->d_wrange) CU_TRY(cudaMalloc(&c->d_wrange, (size_t)c->count * sizeof(uint2)));
     LAUNCH_TRY(launch_quantize_som(g, c->d_som, c->count, c->d_a0, c->d_a1, c->d_anorm, c->stream, c->d_wrange));
     c->launches += 1;
@@ -1131,9 +1151,7 @@ int pink_b200_get_som(pink_b200_ctx* c, float* host_som)
     CU_TRY(cudaSetDevice(c->cfg.device));
     int rc = check_status(c);
     if (rc) return rc;
-    CU_TRY(cudaMemcpy2DAsync(host_som + (size_t)c->first * g.P, (size_t)c->stride * g.P * sizeof(float), c->d_som,
-                             (size_t)g.Pp * sizeof(float), (size_t)g.P * sizeof(float), c->count,
-                             cudaMemcpyDeviceToHost, c->stream));
+    CU_TRY(copy_som(c, host_som, cudaMemcpyDeviceToHost));
     CU_TRY(cudaStreamSynchronize(c->stream));
     return PINK_B200_OK;
 }
@@ -1295,10 +1313,10 @@ static int map_chunk(pink_b200_ctx* c, const float* d_images, uint32_t m, float*
         int rc = ensure_filter_buffers(c, c->map_batch);
         if (rc) return rc;
         // the rotation kernel also writes the estimate's TF32 planes and norms of the transforms
-        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, g.nd * g.nd, c->d_b0, c->d_bf_hi,
+        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, g.Pc, c->d_b0, c->d_bf_hi,
                                  c->d_bf_norm, c->stream, nullptr, c->d_bf_lo));
     } else {
-        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, g.nd * g.nd, c->d_b0, c->d_b1, c->d_bnorm, c->stream));
+        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, g.Pc, c->d_b0, c->d_b1, c->d_bnorm, c->stream));
     }
     DistanceArgs da{};
     da.a0 = c->d_a0; da.a1 = c->d_a1; da.anorm = c->d_anorm; da.n = c->count;
@@ -1616,7 +1634,8 @@ int pink_b200_op_quantize_som(const pink_b200_config* cfg, const float* dev_som,
     Geometry g{};
     int rc = geometry_from_config(cfg, &g);
     if (rc) return rc;
-    if (g.P != g.Pp) return fail(PINK_B200_EINVAL, "this entry needs a neuron size that is a multiple of 4 floats");
+    if (g.P % 4 != 0) return fail(PINK_B200_EINVAL, "this entry needs a neuron size that is a multiple of 4 floats");
+    g.Pc = g.nd * g.nd; g.Pp = g.P;                  // the caller's map is dense
     LAUNCH_TRY(launch_quantize_som(g, dev_som, n_neurons, dev_a0, dev_a1, dev_anorm, static_cast<cudaStream_t>(stream)));
     return PINK_B200_OK;
 }

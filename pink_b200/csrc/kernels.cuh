@@ -27,7 +27,10 @@ struct Geometry
     uint32_t R, T, q;           // rotations, transforms, rotations per quadrant (R/4, 0 when R == 1)
     uint32_t flip;
     uint32_t off;               // crop offset uint32((nd - ed) * 0.5)
-    uint32_t P, Pp;             // neuron size and its row stride in floats (multiple of 4)
+    uint32_t P;                 // neuron size
+    uint32_t Pc, Pp;            // floats from one channel plane to the next in the map and in the base rotations of a context
+                                //   (nd * nd rounded up to 4: planes of any size are 16-byte aligned bulk copies), and from
+                                //   one neuron (base rotation) to the next: C * Pc
     uint32_t K, Kp;             // distance length and operand row stride in ELEMENTS:
                                 //   integer modes: multiple of 128 (bytes per plane row)
                                 //   float mode:    multiple of 16 floats

@@ -41,7 +41,7 @@ quantize_som_kernel(Geometry g, const float* __restrict__ som, void* __restrict_
     __shared__ uint32_t lo_s[8], hi_s[8];
     const size_t n = blockIdx.x;
     const float* src = som + n * g.Pp;
-    const uint32_t P1 = g.nd * g.nd, K1 = g.ed * g.ed;
+    const uint32_t K1 = g.ed * g.ed;
     const uint32_t groups = (g.K + 3) / 4;
     unsigned long long acc = 0;
     for (uint32_t k4 = threadIdx.x; k4 < groups; k4 += blockDim.x) {
@@ -53,7 +53,7 @@ quantize_som_kernel(Geometry g, const float* __restrict__ som, void* __restrict_
             if (k < g.K) {
                 uint32_t c = k / K1, r = k - c * K1;
                 uint32_t i = r / g.ed, jj = r - i * g.ed;
-                if (in_region(g, i, jj)) val[e] = src[c * P1 + (g.off + i) * g.nd + g.off + jj];
+                if (in_region(g, i, jj)) val[e] = src[c * g.Pc + (g.off + i) * g.nd + g.off + jj];
             }
         }
         if (MODE == kModeU8) {
@@ -83,9 +83,11 @@ quantize_som_kernel(Geometry g, const float* __restrict__ som, void* __restrict_
         // bit patterns of min |w| and max |w| over the whole neuron (integer order = float order for
         // non-negative values; NaN patterns compare highest)
         uint32_t lo = 0xFFFFFFFFu, hi = 0;
-        for (uint32_t i = threadIdx.x; i < g.P; i += blockDim.x) {
-            const uint32_t b = __float_as_uint(src[i]) & 0x7FFFFFFFu;
-            lo = min(lo, b); hi = max(hi, b);
+        for (uint32_t c = 0; c < g.C; ++c) {
+            for (uint32_t i = threadIdx.x; i < g.nd * g.nd; i += blockDim.x) {
+                const uint32_t b = __float_as_uint(src[c * g.Pc + i]) & 0x7FFFFFFFu;
+                lo = min(lo, b); hi = max(hi, b);
+            }
         }
         lo = __reduce_min_sync(0xffffffffu, lo); hi = __reduce_max_sync(0xffffffffu, hi);
         if ((threadIdx.x & 31) == 0) { lo_s[threadIdx.x >> 5] = lo; hi_s[threadIdx.x >> 5] = hi; }

@@ -217,8 +217,8 @@ train_steps_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
 
     // ---- constants of the update phase (consumer threads: warps 1..15) ---------------------------
     const uint32_t cwarp = warp - 1, ctid = threadIdx.x - 32;
-    const uint32_t nd = g.nd, P1 = g.nd * g.nd, K1 = g.ed * g.ed;
-    const uint32_t plane_bytes = P1 * 4;
+    const uint32_t nd = g.nd, K1 = g.ed * g.ed;
+    const uint32_t plane_bytes = g.Pc * 4;         // (padding travels along and stays as it is)
     const uint32_t ntask = pl.col_chunks * pl.row_blocks;
     uint32_t tk_si[kMaxTasks], tk_x0[kMaxTasks], tk_y[kMaxTasks], tk_full[kMaxTasks], tk_tail[kMaxTasks];
 #pragma unroll
@@ -556,7 +556,7 @@ train_steps_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
         __syncthreads();
         stamp(a, img, 3, 0);
         const uint32_t M = sh.n_entries;
-        const float* base_img = a.base + (size_t)img * (g.q ? g.q : 1) * g.P;
+        const float* base_img = a.base + (size_t)img * (g.q ? g.q : 1) * g.Pp;
 
         if (warp == 0) {
             // ------------------------------------------------------------ producer --
@@ -566,8 +566,8 @@ train_steps_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
                 uint8_t* st = region + (size_t)s * pl.upd_stage_bytes;
                 const Entry& e = sh.entries[jx];
                 mbar_expect_tx(&sh.upd_full[s], 2 * plane_bytes);
-                bulk_load(st, a.som + (size_t)e.n * g.Pp + (size_t)e.c * P1, plane_bytes, &sh.upd_full[s]);
-                bulk_load(st + pl.upd_off_base, base_img + ((size_t)e.tq * g.C + e.c) * P1, plane_bytes, &sh.upd_full[s]);
+                bulk_load(st, a.som + (size_t)e.n * g.Pp + (size_t)e.c * g.Pc, plane_bytes, &sh.upd_full[s]);
+                bulk_load(st + pl.upd_off_base, base_img + ((size_t)e.tq * g.C + e.c) * g.Pc, plane_bytes, &sh.upd_full[s]);
             };
             if (lane == 0)
                 for (uint32_t jx = 0; jx < M && jx < pl.upd_stages; ++jx) issue(jx);
@@ -596,7 +596,7 @@ train_steps_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
                 uint8_t* st = region + (size_t)s * pl.upd_stage_bytes;
                 if (lane == 0) {
                     if (changed) {
-                        bulk_store(a.som + (size_t)e.n * g.Pp + (size_t)e.c * P1, st, plane_bytes);
+                        bulk_store(a.som + (size_t)e.n * g.Pp + (size_t)e.c * g.Pc, st, plane_bytes);
                         bulk_commit();
                     }
                     if (e.last && neuron_changed) {
@@ -762,14 +762,13 @@ bool step_plan(const Geometry& g, uint32_t n_local, uint32_t n_global, StepPlan*
     const char* dummy = "";
     if (!why_not) why_not = &dummy;
     if (g.mode != kModeU8 && g.mode != kModeU16) { *why_not = "float distances"; return false; }
-    const uint32_t P1 = g.nd * g.nd, K1 = g.ed * g.ed;
-    if ((P1 & 3u) != 0 || g.P != g.Pp) { *why_not = "neuron planes are not a multiple of 16 bytes"; return false; }
+    const uint32_t K1 = g.ed * g.ed;
     if (g.mode == kModeU16 && n_global >= 65536u) { *why_not = "more than 65535 neurons with uint16 distances"; return false; }
     if (n_local == 0) { *why_not = "empty shard"; return false; }
     const uint32_t max_n = g.mode == kModeU8 ? 256u : 128u, planes = g.mode == kModeU8 ? 1u : 2u;
 
     // update phase: stages of {neuron plane, base rotation plane}
-    const uint32_t plane = round_up_u32(P1 * 4, 128);
+    const uint32_t plane = round_up_u32(g.Pc * 4, 128);
     pl->upd_stage_bytes = 2 * plane;
     pl->upd_off_base = plane;
     pl->upd_stages = std::min<uint32_t>(kUpdMax, kRegionBudget / pl->upd_stage_bytes);

@@ -127,9 +127,9 @@ update_kernel(const __grid_constant__ Geometry g, const __grid_constant__ Update
     const UpdateItem it = a.items[blockIdx.y];
     const uint32_t c = blockIdx.x / strips, xs = (blockIdx.x - c * strips) * kStripRows;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t nd = g.nd, ed = g.ed, P1 = nd * nd, K1 = ed * ed;
-    const float* __restrict__ base = a.base + (size_t)it.tq * g.P + (size_t)c * P1;
-    float* w = a.som + (size_t)it.n * g.Pp + (size_t)c * P1;
+    const uint32_t nd = g.nd, ed = g.ed, K1 = ed * ed;
+    const float* __restrict__ base = a.base + (size_t)it.tq * g.Pp + (size_t)c * g.Pc;
+    float* w = a.som + (size_t)it.n * g.Pp + (size_t)c * g.Pc;
     uint8_t* row0 = static_cast<uint8_t*>(a.a0) + ((size_t)it.n * g.Kp + (size_t)c * K1) * (MODE == kModeF32 ? 4 : 1);
     uint8_t* row1 = MODE == kModeU16 ? static_cast<uint8_t*>(a.a1) + (size_t)it.n * g.Kp + (size_t)c * K1 : nullptr;
     const uint32_t x0 = xs + (lane >> 3);
@@ -307,7 +307,7 @@ update_pipe_kernel(Geometry g, UpdateArgs a, PipeParams pp, BmuArgs b)
     if (keys_prefetched) load_keys(4 * (threadIdx.x - 32));
     fence_async_smem();                   // zeroed operand staging visible to later bulk stores
     __syncthreads();
-    const uint32_t plane_bytes = g.P * 4;
+    const uint32_t plane_bytes = g.Pp * 4;
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer --
@@ -317,7 +317,7 @@ update_pipe_kernel(Geometry g, UpdateArgs a, PipeParams pp, BmuArgs b)
             uint8_t* st = pipe_dyn + (size_t)s * pp.stage_bytes;
             mbar_expect_tx(&full_bar[s], 2 * plane_bytes);
             bulk_load(st, a.som + (size_t)items[jx].n * g.Pp, plane_bytes, &full_bar[s]);
-            bulk_load(st + pp.off_base, a.base + (size_t)items[jx].tq * g.P, plane_bytes, &full_bar[s]);
+            bulk_load(st + pp.off_base, a.base + (size_t)items[jx].tq * g.Pp, plane_bytes, &full_bar[s]);
         };
         if (lane == 0)
             for (uint32_t jx = 0; jx < m_fixed; ++jx) issue(jx);
@@ -376,7 +376,7 @@ update_pipe_kernel(Geometry g, UpdateArgs a, PipeParams pp, BmuArgs b)
     } else {
         // ----------------------------------------------------------- consumers --
         const uint32_t cwarp = warp - 1, ctid = threadIdx.x - 32;
-        const uint32_t P1 = g.nd * g.nd, K1 = g.ed * g.ed;
+        const uint32_t K1 = g.ed * g.ed;
         // Update tasks of this thread (the same for every neuron): channel c, column y, rows
         // [x0, x0 + 3 * full + tail).  Idle lanes and tasks get an empty range.
         const uint32_t tasks_per_channel = pp.col_chunks * pp.row_blocks, ntask = g.C * tasks_per_channel;
@@ -392,7 +392,7 @@ update_pipe_kernel(Geometry g, UpdateArgs a, PipeParams pp, BmuArgs b)
             const uint32_t nrows = live ? min(pp.rows_per_block, g.nd - x0) : 0;
             tk_c[k] = c; tk_y[k] = y; tk_x0[k] = x0;
             tk_full[k] = nrows / kPipeUnroll; tk_tail[k] = nrows - tk_full[k] * kPipeUnroll;
-            tk_si[k] = c * P1 + x0 * g.nd + y;
+            tk_si[k] = c * g.Pc + x0 * g.nd + y;
         }
         // Operand units of this thread: within a segment of 128 consecutive operand elements, lane l
         // of a warp converts elements l, l + 32, l + 64, l + 96, so that every shared-memory read of a
@@ -408,7 +408,7 @@ update_pipe_kernel(Geometry g, UpdateArgs a, PipeParams pp, BmuArgs b)
                 const uint32_t kk = (unit / 32) * 128 + (unit % 32) + 32 * e;
                 const uint32_t c = kk / K1, rem = kk - c * K1, ci = rem / g.ed, cj = rem - ci * g.ed;
                 const bool ok = unit < nunit && kk < g.K && in_region(g, ci, cj);   // outside a circular region: stays zero
-                un_src[k][e] = ok ? 4 * (c * P1 + (g.off + ci) * g.nd + g.off + cj) : 0u;   // byte offset in the neuron
+                un_src[k][e] = ok ? 4 * (c * g.Pc + (g.off + ci) * g.nd + g.off + cj) : 0u;   // byte offset in the neuron
                 un_dst[k][e] = ok ? kk : ~0u;
             }
         }
@@ -612,7 +612,7 @@ update_pipe_kernel(Geometry g, UpdateArgs a, PipeParams pp, BmuArgs b)
 #pragma unroll
             for (int k = 0; k < kPipeMaxTasks; ++k) {
                 uint32_t aw = som_a + tk_si[k] * 4;
-                uint32_t ab = base_a + 4 * (uint32_t)((int32_t)(tk_c[k] * P1) + it.ax * (int32_t)tk_x0[k] + it.a0 + it.ay * (int32_t)tk_y[k]);
+                uint32_t ab = base_a + 4 * (uint32_t)((int32_t)(tk_c[k] * g.Pc) + it.ax * (int32_t)tk_x0[k] + it.a0 + it.ay * (int32_t)tk_y[k]);
                 for (uint32_t i = 0; i < tk_full[k]; ++i) {
                     float w[kPipeUnroll], rv[kPipeUnroll], e[kPipeUnroll];
 #pragma unroll
@@ -740,16 +740,16 @@ constexpr size_t kPipeBudget = 216 * 1024;   // of the 227 KB a block may use; t
 size_t pipe_stage_bytes(const Geometry& g)
 {
     const size_t crop = g.mode == kModeF32 ? (size_t)g.Kp * 4 : (g.mode == kModeU16 ? (size_t)g.Kp * 2 : g.Kp);
-    const size_t plane = ((size_t)g.P * 4 + 127) & ~size_t(127);
+    const size_t plane = ((size_t)g.Pp * 4 + 127) & ~size_t(127);
     return 2 * plane + ((crop + 127) & ~size_t(127));
 }
 
-// The pipelined kernel needs bulk-copyable planes (16-byte multiples), at least two
+// The pipelined kernel needs at least two
 // stages of {neuron, base rotation, operand rows} in shared memory, and every
 // consumer thread keeps its tasks and operand units in registers.
 bool pipe_eligible(const Geometry& g)
 {
-    if ((g.P & 3) != 0 || g.P != g.Pp || pipe_stage_bytes(g) * 2 > kPipeBudget || device_sm_count() <= 0) return false;
+    if (pipe_stage_bytes(g) * 2 > kPipeBudget || device_sm_count() <= 0) return false;
     const uint32_t chunks = (g.nd + 31) / 32;
     const uint32_t units = ((g.K + 127) / 128) * 32;
     return g.C * chunks <= (uint32_t)(kPipeMaxTasks * kPipeConsumerWarps) && units <= (uint32_t)(kPipeMaxUnits * kPipeConsumers);
@@ -761,7 +761,7 @@ cudaError_t update_dispatch(const Geometry& g, const UpdateArgs& a, const BmuArg
     if (!fused) return update_classic<MODE>(g, a, st);
     if (!pipe_eligible(g)) return cudaErrorInvalidValue;
     const size_t crop = MODE == kModeF32 ? (size_t)g.Kp * 4 : (MODE == kModeU16 ? (size_t)g.Kp * 2 : g.Kp);
-    const size_t plane = ((size_t)g.P * 4 + 127) & ~size_t(127);
+    const size_t plane = ((size_t)g.Pp * 4 + 127) & ~size_t(127);
     const size_t stage = pipe_stage_bytes(g), budget = kPipeBudget;
     const int sms = device_sm_count();
     PipeParams pp{};

@@ -129,6 +129,37 @@ def test_split_update_bit_exact(cuda, case, mode):
         assert np.array_equal(ctx.get_som(som0).view(np.uint32), want.view(np.uint32))
 
 
+@pytest.mark.parametrize("case", [(1, 20, 7, 5, 0), (1, 64, 45, 31, 0), (2, 50, 35, 35, 1), (3, 40, 27, 19, 0), (4, 30, 21, 14, 0)])
+@pytest.mark.parametrize("mode", [2, 1])
+def test_odd_neuron_sides(cuda, case, mode):
+    """Channel planes whose size is no multiple of four floats are padded on the device: the map goes in and comes out
+    unchanged, the persistent kernel takes them (one launch per batch), and it and the two-kernel path give the oracle's map."""
+    import pink_b200.capi as capi
+    C_, idim, nd, ed, shape = case
+    N, R, n = 20, 8, 5
+    rng = np.random.default_rng(nd * 10 + C_ + mode)
+    som0 = rng.random((N, C_, nd, nd), dtype=np.float32)
+    imgs = blob_images(n, idim, C_, seed=nd).reshape(n, C_, idim, idim)
+    F = O.update_factors(0, 5, 4, O.FUNC_GAUSSIAN, 1.1, 0.2)
+    want = som0.copy()
+    want_bmu = [O.train_step(want, im, F, ed, R, True, mode, shape=shape)[2] for im in imgs]
+    cfg = make_config(capi, N, C_, idim, nd, ed, R, True, mode)
+    cfg.ed_shape = capi.CIRCULAR if shape else capi.QUADRATIC
+    for step_kernel in (0, 1):
+        with Context(capi, cfg, {"step_kernel": step_kernel}) as ctx:
+            ctx.set_som(som0)
+            assert np.array_equal(ctx.get_som(som0).view(np.uint32), som0.view(np.uint32))
+            ctx.set_factors(F)
+            before = ctx.e.launch_count()
+            assert list(ctx.train(imgs)) == want_bmu
+            if step_kernel == 0:
+                assert ctx.e.launch_count() - before < n
+            assert np.array_equal(ctx.get_som(som0).view(np.uint32), want.view(np.uint32))
+            wd, wr = O.map_image(want, imgs[0], ed, R, True, mode, shape=shape)
+            gd, gr = ctx.map(imgs[:1])
+            assert np.array_equal(gr[0], wr) and np.array_equal(gd[0], wd)
+
+
 @pytest.mark.parametrize("case", TRAIN_CASES[:5])
 def test_train_float_mode(cuda, case):
     """float32: one teacher-forced step at a time; the SOM must match the oracle bit for bit whenever
