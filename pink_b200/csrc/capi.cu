@@ -236,6 +236,7 @@ struct pink_b200_ctx
     // and of one mapping batch of transforms, the estimate matrix and the pass's counters
     float* d_af_hi = nullptr; float* d_af_lo = nullptr; float* d_af_norm = nullptr; bool af_valid = false;
     float* d_bf_hi = nullptr; float* d_bf_lo = nullptr; float* d_bf_norm = nullptr; float* d_est = nullptr; size_t filter_imgs = 0;
+    float* d_dots = nullptr;          // training: partial dot products of one image, [max_dot_splits][count][T]
     unsigned long long* d_filter_stats = nullptr;     // {exact evaluations, bits of the largest estimate error seen}
     unsigned long long filter_pairs = 0;              // (neuron, transform) pairs estimated so far
     long long opt_exchange_timeout_ms = 20000;
@@ -329,6 +330,12 @@ bool uses_filter(const pink_b200_ctx* c)
 // Bound of the estimate's error relative to |a|^2 + |b|^2 (derived in filter_f32.cu): 3 * K / 16 * 2^-23 + 2^-17
 float filter_eps(uint32_t K) { return (float)(3.0 * K / 16.0 * 1.1920928955078125e-7 + 7.62939453125e-6); }
 
+// Ranges of K the estimate of one image may be split into: their partial products stay within 256 MB.
+uint32_t max_dot_splits(const pink_b200_ctx* c)
+{
+    return (uint32_t)std::min<uint64_t>(kMaxDotSplits, std::max<uint64_t>(1, (1ull << 26) / ((uint64_t)c->count * c->g.T)));
+}
+
 int ensure_filter_buffers(pink_b200_ctx* c, size_t imgs)
 {
     const Geometry& g = c->g;
@@ -414,12 +421,13 @@ int train_step(pink_b200_ctx* c, size_t slot_img, uint32_t* bmu_slot)
         DistanceArgs fa = da;
         fa.a0 = c->d_af_hi; fa.a1 = c->d_af_lo; fa.anorm = c->d_af_norm;
         fa.b0 = c->d_bf_hi; fa.b1 = c->d_bf_lo; fa.bnorm = c->d_bf_norm;
-        fa.s_out = c->d_est;
-        e = launch_distance_tf32(g, fa, c->stream, &why);
+        fa.s_out = c->d_dots;
+        uint32_t splits = max_dot_splits(c);
+        e = launch_dots_tf32(g, fa, &splits, c->stream, &why);
         if (e == cudaSuccess) {
-            why = "refine_f32_kernel launch";
-            e = launch_refine_f32(g, A, c->d_af_norm, c->count, B, c->d_bf_norm, 1, c->d_est, filter_eps(g.K), c->d_keys,
-                                  c->d_filter_stats, c->stream);
+            why = "refine_team_kernel launch";
+            e = launch_refine_f32_dots(g, A, c->d_af_norm, c->count, B, c->d_bf_norm, c->d_dots, splits, filter_eps(g.K), c->d_keys,
+                                       c->d_filter_stats, c->stream);
         }
         c->filter_pairs += (unsigned long long)c->count * g.T;
         c->launches += 3;
@@ -838,6 +846,7 @@ int train_prepare(pink_b200_ctx* c, uint64_t n)
     if (uses_filter(c) && !c->use_steps) {
         int rcf = ensure_filter_buffers(c, c->filter_imgs ? c->filter_imgs : 1);
         if (rcf) return rcf;
+        if (!c->d_dots) CU_TRY(cudaMalloc(&c->d_dots, (size_t)max_dot_splits(c) * c->g.T * c->count * sizeof(float)));
     }
     if (!c->have_factors) return fail(PINK_B200_ESTATE, "pink_b200_set_update_factors must be called before training");
     if (c->cfg.world_size > 1 && !c->comm)
@@ -1020,7 +1029,7 @@ int pink_b200_destroy(pink_b200_ctx* c)
     free_dev(c->d_cs); free_dev(c->d_sn); free_dev(c->d_factors); free_dev(c->d_coords); free_dev(c->d_lut); free_dev(c->d_base);
     free_dev(c->d_b0); free_dev(c->d_b1); free_dev(c->d_bnorm); free_dev(c->d_keys);
     free_dev(c->d_af_hi); free_dev(c->d_af_lo); free_dev(c->d_af_norm); free_dev(c->d_bf_hi); free_dev(c->d_bf_lo);
-    free_dev(c->d_bf_norm); free_dev(c->d_est); free_dev(c->d_filter_stats);
+    free_dev(c->d_bf_norm); free_dev(c->d_est); free_dev(c->d_dots); free_dev(c->d_filter_stats);
     free_dev(c->d_items); free_dev(c->d_nitems); free_dev(c->d_stats); free_dev(c->d_wrange); free_dev(c->d_rmax);
     free_dev(c->d_circle); free_dev(c->d_owners); free_dev(c->d_ctrl); free_dev(c->d_stamps);
     for (cudaEvent_t e : c->prof_launch_events) cudaEventDestroy(e);

@@ -91,6 +91,7 @@ struct TcParams
     int* status;
     uint32_t n, T, num_kb, n_tile;
     uint32_t swap;              // kModeTf32 only: the transforms are the tile rows (M side), the neurons its columns
+    uint32_t splits, kb_split;  // kModeTf32, one image: 0, or grid z = ranges of kb_split K slices whose raw dot products go to s_out[z]
     uint32_t stages, b_bytes;   // ring depth; bytes of this CTA's transform rows per plane and stage (multiple of 1024)
     uint32_t* tail_counter;     // nullable: block arrival counter (zero between launches) that enables the tail below
     BmuArgs tail;               // the last block to finish reduces the shard's keys to its record and publishes it
@@ -123,7 +124,9 @@ distance_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t m0 = blockIdx.x * kBlockM;
     const uint32_t t0 = blockIdx.y * p.n_tile;
-    const uint32_t img = blockIdx.z;
+    const bool raw = MODE == kModeTf32 && p.splits != 0;
+    const uint32_t img = raw ? 0u : blockIdx.z;
+    const uint32_t kb_lo = raw ? blockIdx.z * p.kb_split : 0u, num_kb = raw ? min(p.kb_split, p.num_kb - kb_lo) : p.num_kb;
     // PAIR: rank of this CTA in its pair (the even CTA issues the MMAs) and the transform rows it stages
     const uint32_t pair_rank = PAIR ? cluster_ctarank() : 0u;
     const uint32_t b_rows = PAIR ? p.n_tile / 2 : p.n_tile;
@@ -159,11 +162,11 @@ distance_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
             const int32_t arow = (int32_t)(MODE == kModeTf32 && p.swap ? img * p.T + m0 : m0);
             const int32_t brow = (int32_t)(MODE == kModeTf32 && p.swap ? t0 + pair_rank * b_rows
                                                                       : img * p.T + t0 + pair_rank * b_rows);
-            for (uint32_t kb = 0; kb < p.num_kb; ++kb) {
+            for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 const uint32_t s = kb % p.stages, ph = (kb / p.stages) & 1;
                 if (!mbar_wait(&empty_bar[s], ph ^ 1)) { report(p.status, kDevTimeoutProducer); break; }
                 uint8_t* st = ring + s * stage_bytes;
-                const int32_t kx = (int32_t)(kb * kBlockK);
+                const int32_t kx = (int32_t)((kb_lo + kb) * kBlockK);
                 if (PAIR) {
                     const uint32_t bar = map_to_cta(smem_u32(&full_bar[s]), 0);      // the issuing CTA's barrier
                     mbar_expect_tx_cluster(bar, stage_tx);
@@ -204,7 +207,7 @@ distance_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
                 }
             };
             bool ok = true;
-            for (uint32_t kb = 0; kb < p.num_kb && ok; ++kb) {
+            for (uint32_t kb = 0; kb < num_kb && ok; ++kb) {
                 const uint32_t s = kb % p.stages, ph = (kb / p.stages) & 1;
                 if (!mbar_wait(&full_bar[s], ph)) { report(p.status, kDevTimeoutMma); ok = false; break; }
                 tc_fence_after();
@@ -257,11 +260,11 @@ distance_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
         const uint32_t ncols = n_cols > t0 ? min(p.n_tile, n_cols - t0) : 0u;     // columns of this tile that exist
         for (uint32_t j = et; j < p.n_tile; j += 128) {
             val_t v = 0;
-            if (j < ncols) v = swapped ? static_cast<const val_t*>(p.anorm)[t0 + j]
+            if (j < ncols && !raw) v = swapped ? static_cast<const val_t*>(p.anorm)[t0 + j]
                                        : static_cast<const val_t*>(p.bnorm)[(size_t)img * p.T + t0 + j];
             nbv[j] = v;
         }
-        const val_t na = n >= m_rows ? val_t(0) : swapped ? static_cast<const val_t*>(p.bnorm)[(size_t)img * p.T + n]
+        const val_t na = n >= m_rows || raw ? val_t(0) : swapped ? static_cast<const val_t*>(p.bnorm)[(size_t)img * p.T + n]
                                                           : static_cast<const val_t*>(p.anorm)[n];
         asm volatile("bar.sync 1, 128;" ::: "memory");      // nbv visible to the four epilogue warps
 
@@ -288,7 +291,17 @@ distance_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
             };
             auto reduce = [&](uint32_t c0, const uint32_t (&x0)[16], const uint32_t (&x1)[16], const uint32_t (&x2)[16]) {
                 val_t sv[16];
-                if (MODE == kModeTf32) {
+                if (raw) {
+                    // partial dot products of this K range: the kernel that sums them adds the norms
+                    float* dst = static_cast<float*>(p.s_out) + (size_t)blockIdx.z * p.n * p.T;
+                    const size_t row_step = swapped ? 1 : p.T, col_step = swapped ? p.T : 1;
+                    if (n < m_rows) {
+#pragma unroll
+                        for (uint32_t j = 0; j < 16; ++j)
+                            if (c0 + j < ncols)
+                                dst[n * row_step + (t0 + c0 + j) * col_step] = __uint_as_float(x0[j]) + __uint_as_float(x1[j]);
+                    }
+                } else if (MODE == kModeTf32) {
                     // the estimate of every pair goes out (row-major per neuron: 64 contiguous bytes per thread
                     // and chunk); nothing is reduced here
                     if (swapped) {
@@ -412,7 +425,7 @@ distance_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
 // ------------------------------------------------------------------ host side --
 
 template <int MODE, bool PAIR>
-cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st, const char** why, bool swap = false)
+cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st, const char** why, bool swap = false, uint32_t* splits = nullptr)
 {
     using Cfg = TcCfg<MODE, PAIR>;
     using L = SmemLayout<MODE, PAIR>;
@@ -437,8 +450,32 @@ cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st,
         if (sms > 0 && rows * tiles < (uint64_t)sms)
             tiles = (uint32_t)std::max<uint64_t>(tiles, std::min<uint64_t>(most, (uint64_t)sms / rows));   // one wave
     }
-    uint32_t n_tile = ((n_extent + tiles - 1) / tiles + 15) & ~15u;
-    if (n_tile > Cfg::max_n) n_tile = Cfg::max_n;
+    auto tile_width = [&](uint32_t count) { return std::min<uint32_t>(Cfg::max_n, ((n_extent + count - 1) / count + 15) & ~15u); };
+    const uint32_t slices = (uint32_t)((MODE == kModeTf32 ? 4ull : 1ull) * g.Kp / kBlockK);
+    uint32_t kb_split = slices;
+    if (splits) {
+        // One image's tiles alone leave most SMs idle or, narrow, make every SM pull the whole row tile (400 x 720 x 4096:
+        // 54 blocks of 5 MB, 40.6 us; now 16.6).  With K split too, the choice of column tiles and K ranges that
+        // moves the fewest bytes per SM: operand slices in, partial products out and in again.
+        const uint32_t max_splits = std::min(std::max(*splits, 1u), kMaxDotSplits);
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const uint64_t wave = sms > 0 ? sms : 148;
+        uint64_t best = ~0ull;
+        const uint32_t fewest = (n_extent + Cfg::max_n - 1) / Cfg::max_n, most = std::max<uint32_t>(fewest, n_extent / 32);
+        for (uint32_t count = fewest; count <= most; ++count) {
+            const uint32_t width = tile_width(count), columns = (n_extent + width - 1) / width, b = PAIR ? width / 2 : width;
+            for (uint32_t s = 1; s <= max_splits && (s == 1 || 2 * s <= slices); ++s) {
+                const uint64_t blocks = (uint64_t)m_tiles * columns * s, waves = (blocks + wave - 1) / wave;
+                const uint32_t len = (slices + s - 1) / s;
+                if ((s - 1) * len >= slices) continue;                // (the last range would be empty)
+                const uint64_t cost = waves * len * (kBlockM + b) * kBlockK * Cfg::planes + (uint64_t)s * a.n * g.T * 8 / wave;
+                if (cost < best) { best = cost; tiles = count; *splits = s; kb_split = len; }
+            }
+        }
+    }
+    const uint32_t n_tile = tile_width(tiles);
     const uint32_t n_tiles = (n_extent + n_tile - 1) / n_tile;
     const uint32_t b_box = PAIR ? n_tile / 2 : n_tile;         // column-side rows one CTA stages per K slice
 
@@ -467,7 +504,7 @@ cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st,
     const uint32_t b_bytes = (b_box * kBlockK + 1023) & ~1023u;
     const uint32_t stage_bytes = Cfg::planes * (L::a_bytes + b_bytes);
     const uint32_t num_kb = (uint32_t)(row_bytes / kBlockK);
-    uint32_t stages = std::max(2u, std::min(std::min(kMaxStages, L::ring_budget / stage_bytes), num_kb));
+    uint32_t stages = std::max(2u, std::min(std::min(kMaxStages, L::ring_budget / stage_bytes), kb_split));
     {
         // More blocks than SMs (mapping: a batch of images per launch): a ring of three stages is as good as a deeper
         // one when a second block of the same kernel shares the SM -- one block's epilogue and first loads then hide
@@ -487,10 +524,11 @@ cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st,
     p.anorm = a.anorm; p.bnorm = a.bnorm; p.keys = a.keys; p.s_out = a.s_out; p.status = a.status;
     p.n = a.n; p.T = g.T; p.num_kb = num_kb; p.n_tile = n_tile; p.swap = swap ? 1u : 0u;
     p.stages = stages; p.b_bytes = b_bytes;
+    p.splits = splits ? *splits : 0u; p.kb_split = kb_split;
     p.tail_counter = a.tail ? a.tail_counter : nullptr;
     if (a.tail) p.tail = *a.tail;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(m_tiles, n_tiles, a.n_img);
+    cfg.gridDim = dim3(m_tiles, n_tiles, splits ? *splits : a.n_img);
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = L::ring_off + stages * stage_bytes + L::slack;
     cfg.stream = st;
@@ -524,7 +562,7 @@ cudaError_t launch_distance_f32(const Geometry& g, const DistanceArgs& a, cudaSt
 
 // float32 filter pass: a0/a1 and b0/b1 are the TF32 word planes (high, low) of the operands, anorm/bnorm float
 // |.|^2, s_out [n_img][n][T] float receives the estimates; keys are not touched.  Needs Kp % 32 == 0.
-cudaError_t launch_distance_tf32(const Geometry& g, const DistanceArgs& a, cudaStream_t st, const char** why)
+static cudaError_t estimate_tf32(const Geometry& g, const DistanceArgs& a, uint32_t* splits, cudaStream_t st, const char** why)
 {
     *why = "";
     if (a.n == 0 || a.n_img == 0) return cudaSuccess;
@@ -538,8 +576,19 @@ cudaError_t launch_distance_tf32(const Geometry& g, const DistanceArgs& a, cudaS
     };
     const bool swap = padded(g.T, a.n) < padded(a.n, g.T);
     const uint32_t m_extent = swap ? g.T : a.n;
-    if (m_extent > kBlockM && !a.single_cta) return launch_tc<kModeTf32, true>(g, a, st, why, swap);
-    return launch_tc<kModeTf32, false>(g, a, st, why, swap);
+    if (m_extent > kBlockM && !a.single_cta) return launch_tc<kModeTf32, true>(g, a, st, why, swap, splits);
+    return launch_tc<kModeTf32, false>(g, a, st, why, swap, splits);
+}
+
+cudaError_t launch_distance_tf32(const Geometry& g, const DistanceArgs& a, cudaStream_t st, const char** why)
+{
+    return estimate_tf32(g, a, nullptr, st, why);
+}
+
+cudaError_t launch_dots_tf32(const Geometry& g, const DistanceArgs& a, uint32_t* splits, cudaStream_t st, const char** why)
+{
+    if (a.n_img > 1) { *why = "launch_dots_tf32: one image"; return cudaErrorInvalidValue; }
+    return estimate_tf32(g, a, splits, st, why);
 }
 
 bool distance_has_tail(const Geometry& g) { return g.mode == kModeU8 || g.mode == kModeU16; }

@@ -19,6 +19,8 @@
 //   addition may lose one unit in the last place of the running sum even if the unit truncates (observed: it
 //   does).  Even and odd K steps use separate accumulators, so an accumulator sees 3 * K / 16 additions of its own
 //   part of the sum: 3 * K / 16 * 2^-23 of the whole.
+// (Training splits K into up to 16 ranges of at least two slices, whose partial sums are added in float: an accumulator then
+// sees a range's share of those additions, and the fewer than 16 roundings of half a unit that join the ranges are less.)
 // eps = 3 * K / 16 * 2^-23 + 2^-17.  The largest deviation seen among the evaluated pairs is recorded so that tests
 // can compare it with eps (C2: 0.3 of eps).
 #include "kernels.cuh"
@@ -142,6 +144,85 @@ refine_f32_kernel(const float* __restrict__ A, const float* __restrict__ anorm, 
     }
 }
 
+// One block per neuron of one image: the same selection and the same exact sums (lane by lane in the same order, so both
+// kernels give the same bits), but the block's warps share the scan of the estimates and form the exact sums of
+// different transforms at the same time.  A training step has one image's pairs only: as one warp per neuron they
+// filled a fifteenth of the GPU and every candidate's 2 x Kp floats were a chain of load latencies of its own.
+// 400 neurons x 720 transforms x 4096: 48.3 -> 13.9 us an image.  `dots` holds `splits` partial dot products of every pair
+// ([splits][n][T], see launch_dots_tf32); adding them up costs splits - 1 roundings, fewer than the running sums
+// inside the tensor core lose by being shorter.  Shared memory: T estimates, then a list of T 16-bit indices.
+__global__ void __launch_bounds__(kRefineWarps * 32, 3)
+refine_team_kernel(const float* __restrict__ A, const float* __restrict__ anorm, uint32_t n, const float* __restrict__ B,
+                   const float* __restrict__ bnorm, uint32_t T, uint32_t Kp, const float* __restrict__ dots, uint32_t splits,
+                   float eps, unsigned long long* __restrict__ keys, unsigned long long* __restrict__ stats)
+{
+    extern __shared__ float est_s[];
+    uint16_t* list = reinterpret_cast<uint16_t*>(est_s + T);
+    __shared__ float ub_s[kRefineWarps], worst_s[kRefineWarps];
+    __shared__ unsigned long long key_s[kRefineWarps];
+    __shared__ uint32_t count_s;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nn = blockIdx.x;
+    const float na = anorm[nn];
+    if (tid == 0) count_s = 0;
+    float ub = __int_as_float(0x7f800000);
+    unsigned long long first = kKeyEmpty;
+    for (uint32_t t = tid; t < T; t += kRefineWarps * 32) {
+        float dot = 0.0f;
+        for (uint32_t s = 0; s < splits; ++s) dot += dots[((size_t)s * n + nn) * T + t];
+        const float sum = __fadd_rn(na, bnorm[t]), v = fmaxf(sum - 2.0f * dot, 0.0f);
+        est_s[t] = v;
+        ub = fminf(ub, __fadd_rn(v, __fmul_rn(eps, sum)));
+        const unsigned long long k = ((unsigned long long)__float_as_uint(v) << 32) | t;
+        first = k < first ? k : first;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        ub = fminf(ub, __shfl_xor_sync(0xffffffffu, ub, o));
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, first, o);
+        first = other < first ? other : first;
+    }
+    if (lane == 0) { ub_s[warp] = ub; key_s[warp] = first; }
+    __syncthreads();
+    for (uint32_t w = 0; w < kRefineWarps; ++w) { ub = fminf(ub, ub_s[w]); first = key_s[w] < first ? key_s[w] : first; }
+    const uint32_t t_first = (uint32_t)(first & 0xffffffffu);     // evaluated in any case
+
+    for (uint32_t t = tid; t < T; t += kRefineWarps * 32)
+        if (t == t_first || __fsub_rn(est_s[t], __fmul_rn(eps, __fadd_rn(na, bnorm[t]))) <= ub)
+            list[atomicAdd(&count_s, 1u)] = (uint16_t)t;
+    __syncthreads();
+    const uint32_t count = count_s;
+
+    const float4* a4 = reinterpret_cast<const float4*>(A + (size_t)nn * Kp);
+    unsigned long long best = kKeyEmpty;
+    float worst = 0.0f;
+    for (uint32_t c = warp; c < count; c += kRefineWarps) {
+        const uint32_t t = list[c];
+        const float4* b4 = reinterpret_cast<const float4*>(B + (size_t)t * Kp);
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll 8
+        for (uint32_t i = lane; i < Kp / 4; i += 32) {
+            const float4 x = __ldg(a4 + i), y = __ldg(b4 + i);
+            const float d0 = x.x - y.x, d1 = x.y - y.y, d2 = x.z - y.z, d3 = x.w - y.w;
+            s0 = fmaf(d0, d0, s0); s1 = fmaf(d1, d1, s1); s2 = fmaf(d2, d2, s2); s3 = fmaf(d3, d3, s3);
+        }
+        float s = (s0 + s1) + (s2 + s3);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const unsigned long long key = ((unsigned long long)__float_as_uint(s) << 32) | t;
+        best = key < best ? key : best;
+        worst = fmaxf(worst, fabsf(est_s[t] - s) / fmaxf(na + bnorm[t], 1e-30f));
+    }
+    __syncthreads();                                      // key_s has been read
+    if (lane == 0) { key_s[warp] = best; worst_s[warp] = worst; }
+    __syncthreads();
+    if (tid == 0) {
+        for (uint32_t w = 1; w < kRefineWarps; ++w) { best = key_s[w] < best ? key_s[w] : best; worst = fmaxf(worst, worst_s[w]); }
+        keys[nn] = best;
+        if (stats) {
+            atomicAdd(&stats[0], (unsigned long long)count);
+            atomicMax(&stats[1], (unsigned long long)__float_as_uint(worst));
+        }
+    }
+}
+
 } // namespace
 
 cudaError_t launch_split_tf32(const float* src, uint64_t rows, uint32_t Kp, float* hi, float* lo, float* norm, cudaStream_t st)
@@ -169,6 +250,25 @@ cudaError_t launch_refine_f32(const Geometry& g, const float* A, const float* an
     }
     dim3 grid((n + kRefineWarps - 1) / kRefineWarps, n_img);
     refine_f32_kernel<<<grid, kRefineWarps * 32, smem, st>>>(A, anorm, n, B, bnorm, g.T, g.Kp, est, eps, keys, stats);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_refine_f32_dots(const Geometry& g, const float* A, const float* anorm, uint32_t n, const float* B, const float* bnorm,
+                                   const float* dots, uint32_t splits, float eps, unsigned long long* keys,
+                                   unsigned long long* stats, cudaStream_t st)
+{
+    if (n == 0) return cudaSuccess;
+    const size_t smem = (size_t)g.T * (sizeof(float) + sizeof(uint16_t));
+    if (g.T > 65536u || smem > 200u * 1024u || splits == 0) return cudaErrorInvalidValue;
+    static thread_local int attr_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev != attr_dev) {
+        cudaError_t e = cudaFuncSetAttribute(refine_team_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e != cudaSuccess) return e;
+        attr_dev = dev;
+    }
+    refine_team_kernel<<<n, kRefineWarps * 32, smem, st>>>(A, anorm, n, B, bnorm, g.T, g.Kp, dots, splits, eps, keys, stats);
     return cudaGetLastError();
 }
 

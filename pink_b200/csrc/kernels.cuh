@@ -108,6 +108,14 @@ cudaError_t launch_distance(const Geometry& g, const DistanceArgs& a, cudaStream
 // (float bits << 32 | transform) of the first minimum; cand_count (nullable) accumulates the exact evaluations.
 cudaError_t launch_split_tf32(const float* src, uint64_t rows, uint32_t Kp, float* hi, float* lo, float* norm, cudaStream_t st);
 cudaError_t launch_distance_tf32(const Geometry& g, const DistanceArgs& a, cudaStream_t st, const char** why);
+// For one image (training): launch_dots_tf32 leaves the dot products ah.bh + ah.bl + al.bh themselves, in partial sums over
+// ranges of K (a.s_out: [splits][n][T]; *splits: in the most that a.s_out holds, out the number used; norms are not read), and
+// launch_refine_f32_dots adds them up, forms the estimates and goes on as launch_refine_f32.
+constexpr uint32_t kMaxDotSplits = 16;
+cudaError_t launch_dots_tf32(const Geometry& g, const DistanceArgs& a, uint32_t* splits, cudaStream_t st, const char** why);
+cudaError_t launch_refine_f32_dots(const Geometry& g, const float* A, const float* anorm, uint32_t n, const float* B, const float* bnorm,
+                                   const float* dots, uint32_t splits, float eps, unsigned long long* keys,
+                                   unsigned long long* cand_count, cudaStream_t st);
 cudaError_t launch_refine_f32(const Geometry& g, const float* A, const float* anorm, uint32_t n, const float* B, const float* bnorm,
                               uint32_t n_img, const float* est, float eps, unsigned long long* keys,
                               unsigned long long* cand_count, cudaStream_t st);

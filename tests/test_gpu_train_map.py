@@ -160,6 +160,34 @@ def test_odd_neuron_sides(cuda, case, mode):
             assert np.array_equal(gr[0], wr) and np.array_equal(gd[0], wd)
 
 
+@pytest.mark.parametrize("case", [
+    # neurons, C, id, nd, ed, R, flip: one and several tiles on either side, both orientations of the estimate, one K slice
+    # to hundreds (no split, uneven last ranges), transforms that are no multiple of four
+    (1, 1, 12, 6, 5, 1, False), (100, 1, 40, 28, 20, 12, True), (130, 1, 64, 45, 45, 4, False), (257, 2, 40, 28, 27, 360, True),
+    (40, 1, 90, 70, 69, 60, True), (700, 1, 30, 21, 15, 36, False),
+])
+def test_float_step_equals_map(cuda, case):
+    """float32 training selects its best matching unit from the same exact sums, bit for bit, as mapping reports."""
+    import pink_b200.capi as capi
+    N, C_, idim, nd, ed, R, flip = case
+    rng = np.random.default_rng(N + ed)
+    som0 = rng.random((N, C_, nd, nd), dtype=np.float32)
+    imgs = blob_images(3, idim, C_, seed=N).reshape(3, C_, idim, idim) if idim >= 15 else rng.random((3, C_, idim, idim), dtype=np.float32)
+    F = O.update_factors(0, N, 1, O.FUNC_GAUSSIAN, 1.1, 0.2)
+    with Context(capi, make_config(capi, N, C_, idim, nd, ed, R, flip, 0)) as ctx:
+        ctx.set_som(som0)
+        ctx.set_factors(F)
+        for img in imgs:
+            som = ctx.get_som(som0)
+            d, r = ctx.map(img[None])
+            bmu = int(ctx.train(img[None])[0])
+            assert bmu == int(d[0].argmin())
+            got = ctx.get_som(som0)
+            near = O.rotation_set(img, nd, R, flip)[r[0][bmu]]
+            w = som[bmu]
+            assert np.array_equal(got[bmu].view(np.uint32), (w - (w - near) * F[bmu, bmu]).astype(np.float32).view(np.uint32))
+
+
 @pytest.mark.parametrize("case", TRAIN_CASES[:5])
 def test_train_float_mode(cuda, case):
     """float32: one teacher-forced step at a time; the SOM must match the oracle bit for bit whenever
