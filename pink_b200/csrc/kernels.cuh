@@ -243,7 +243,8 @@ constexpr uint32_t kStepStampWords = 12;        // opt-in timeline words per ima
 //   bmu_word[i]: minimum over all (neuron, transform tile) partial minima of image i of
 //                (code << s) | global neuron index, s = 32 (uint8) or 16 (uint16)
 //   bar:         arrival counter of the grid barriers (counts up from 0xFFFFFFFF, i.e. -1)
-struct StepCtrl { unsigned long long bmu_word[kStepBatchMax]; uint32_t bar; uint32_t pad; };
+//   failed:      cleared by a block whose wait expired; read together with bar in one 8-byte load
+struct StepCtrl { unsigned long long bmu_word[kStepBatchMax]; uint32_t bar; uint32_t failed; };
 
 // Launch shape and shared-memory layout, fixed per context.
 struct StepPlan
