@@ -122,7 +122,7 @@ __device__ __forceinline__ bool step_aborted(const StepShared& sh)
 
 // Bounded mbarrier wait that also gives up as soon as this block, or (checked more rarely) any block
 // of any rank of this launch, has failed.
-__device__ __forceinline__ bool step_wait(uint64_t* bar, uint32_t parity, const StepShared& sh, const int* status)
+__device__ __forceinline__ bool step_wait(uint32_t bar, uint32_t parity, const StepShared& sh, const int* status)
 {
     for (uint32_t i = 0; i < kSpinLimit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
@@ -130,6 +130,11 @@ __device__ __forceinline__ bool step_wait(uint64_t* bar, uint32_t parity, const 
         if ((i & 1023u) == 1023u && status && ld_relaxed_gpu_s32(status) != kDevOk) return false;
     }
     return false;
+}
+
+__device__ __forceinline__ bool step_wait(uint64_t* bar, uint32_t parity, const StepShared& sh, const int* status)
+{
+    return step_wait(smem_u32(bar), parity, sh, status);
 }
 
 // Barrier over all blocks of the launch (all are resident: one per SM, cooperative launch).  `target`
@@ -263,24 +268,30 @@ train_steps_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
         stamp(a, img, 0, 0);
         if (warp == 0) {
             // ------------------------------------------------------ TMA producer --
-            if (lane == 0) {
+            // One thread runs this loop and one the next; a slice costs whatever their instructions cost, hence no division by the
+            // ring's depth, no generic addresses and no mapa per slice.  (With them a slice took 630 cycles here and 780
+            // there, however few bytes it had: 100 neurons x 720 x 1024: a distance phase of 5.2 us, now 3.9;
+            // 2791 x 1440 x 4096: 18.9 -> 14.1; uint16, 1600 x 720 x 11250: 64 -> 42.)
+            if (elect_one()) {
                 fence_proxy_async_all();      // operand rows rewritten by the update phase (any block) before these loads
+                const uint32_t ring0 = smem_u32(region), stages = pl.ring_stages;
+                const uint32_t empty0 = smem_u32(&sh.empty_bar[0]);
+                const uint32_t full0 = PAIR ? map_to_cta(smem_u32(&sh.full_bar[0]), 0) : smem_u32(&sh.full_bar[0]);   // the issuing block's barriers
                 uint32_t k = 0;
                 for (uint32_t item = unit; item < n_items && !step_aborted(sh); item += n_units, ++k) {
                     const uint32_t mu = item % pl.m_units, nt = item / pl.m_units;
                     const int32_t m0 = (int32_t)((PAIR ? 2 * mu + pair_rank : mu) * kBlockM);
                     const int32_t brow = (int32_t)(a.b_row0 + img * g.T + nt * pl.n_tile + pair_rank * b_rows);
+                    const uint32_t it0 = (img * my_items + k) * num_kb;
+                    uint32_t s = it0 % stages, ph = (it0 / stages) & 1, st = ring0 + s * ring_stage_bytes;
+                    int32_t kx = 0;
                     // All tiles walk K in the same order from the same slice: the tiles that share neuron rows (or
                     // transform rows) run at the same time on other SMs and then ask for the same L2 lines at about the
                     // same moment, which is cheaper for the L2 than the same requests spread in time (measured both ways).
                     for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                        const uint32_t it = (img * my_items + k) * num_kb + kb;
-                        const uint32_t s = it % pl.ring_stages, ph = (it / pl.ring_stages) & 1;
-                        if (!step_wait(&sh.empty_bar[s], ph ^ 1, sh, a.status)) { step_fail(sh, a.status, kDevTimeoutProducer); break; }
-                        uint8_t* st = region + s * ring_stage_bytes;
-                        const int32_t kx = (int32_t)(kb * kBlockK);
+                        if (!step_wait(empty0 + 8 * s, ph ^ 1, sh, a.status)) { step_fail(sh, a.status, kDevTimeoutProducer); break; }
+                        const uint32_t bar = full0 + 8 * s;
                         if (PAIR) {
-                            const uint32_t bar = map_to_cta(smem_u32(&sh.full_bar[s]), 0);     // the issuing block's barrier
                             mbar_expect_tx_cluster(bar, stage_tx);
                             tma_load_2d_pair(st, &map_a0, bar, kx, m0);
                             tma_load_2d_pair(st + Cfg::planes * a_bytes, &map_b0, bar, kx, brow);
@@ -289,48 +300,50 @@ train_steps_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
                                 tma_load_2d_pair(st + Cfg::planes * a_bytes + pl.b_bytes, &map_b1, bar, kx, brow);
                             }
                         } else {
-                            mbar_expect_tx(&sh.full_bar[s], stage_tx);
-                            tma_load_2d(st, &map_a0, &sh.full_bar[s], kx, m0);
-                            tma_load_2d(st + Cfg::planes * a_bytes, &map_b0, &sh.full_bar[s], kx, brow);
+                            mbar_expect_tx(bar, stage_tx);
+                            tma_load_2d(st, &map_a0, bar, kx, m0);
+                            tma_load_2d(st + Cfg::planes * a_bytes, &map_b0, bar, kx, brow);
                             if (MODE == kModeU16) {
-                                tma_load_2d(st + a_bytes, &map_a1, &sh.full_bar[s], kx, m0);
-                                tma_load_2d(st + Cfg::planes * a_bytes + pl.b_bytes, &map_b1, &sh.full_bar[s], kx, brow);
+                                tma_load_2d(st + a_bytes, &map_a1, bar, kx, m0);
+                                tma_load_2d(st + Cfg::planes * a_bytes + pl.b_bytes, &map_b1, bar, kx, brow);
                             }
                         }
+                        kx += (int32_t)kBlockK;
+                        st += ring_stage_bytes;
+                        if (++s == stages) { s = 0; ph ^= 1; st = ring0; }
                     }
                 }
             }
             __syncwarp();
         } else if (warp == 1) {
             // -------------------------------------------------------- MMA issuer --
-            if (pair_rank == 0 && lane == 0) {
+            if (pair_rank == 0 && elect_one()) {
                 const uint32_t idesc = make_idesc_u8(PAIR ? 2 * kBlockM : kBlockM, pl.n_tile);
                 auto mma = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t acc) {
                     if (PAIR) umma_i8_pair(d, da, db, idesc, acc); else umma_i8(d, da, db, idesc, acc);
                 };
-                auto commit = [&](uint64_t* bar) {
-                    if (PAIR) {
-                        umma_commit_pair(smem_u32(bar));
-                        umma_commit_pair(map_to_cta(smem_u32(bar), 1));
-                    } else {
-                        umma_commit(bar);
-                    }
+                // `off`: byte offset of the barrier from the first empty barrier, in both blocks alike
+                const uint32_t own0 = smem_u32(&sh.empty_bar[0]), peer0 = PAIR ? map_to_cta(own0, 1) : 0u;
+                auto commit = [&](uint32_t off) {
+                    if (PAIR) { umma_commit_pair(own0 + off); umma_commit_pair(peer0 + off); }
+                    else umma_commit(own0 + off);
                 };
+                const uint32_t full0 = smem_u32(&sh.full_bar[0]), ring0 = smem_u32(region), stages = pl.ring_stages;
+                const uint64_t a_hi0 = make_sw128_kmajor_desc(ring0), b_hi0 = make_sw128_kmajor_desc(ring0 + Cfg::planes * a_bytes);
+                const uint64_t to_a_lo = a_bytes >> 4, to_b_lo = pl.b_bytes >> 4;        // from a high-byte descriptor to its low-byte one
                 for (uint32_t k = 0; k < my_items && !step_aborted(sh); ++k) {
                     const uint32_t idn = img * my_items + k;
                     // the epilogue warps (of both blocks of a pair) are done with the previous tile's accumulators
                     if (!step_wait(&sh.tmem_empty, (idn & 1) ^ 1, sh, a.status)) { step_fail(sh, a.status, kDevTimeoutMma); break; }
                     tc_fence_after();
                     bool ok = true;
+                    const uint32_t it0 = idn * num_kb;
+                    uint32_t s = it0 % stages, ph = (it0 / stages) & 1, off = s * (ring_stage_bytes >> 4);
                     for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                        const uint32_t it = idn * num_kb + kb;
-                        const uint32_t s = it % pl.ring_stages, ph = (it / pl.ring_stages) & 1;
-                        if (!step_wait(&sh.full_bar[s], ph, sh, a.status)) { step_fail(sh, a.status, kDevTimeoutMma); ok = false; break; }
-                        if (k == 0 && kb == 0) stamp(a, img, 8, 32);
+                        if (!step_wait(full0 + 8 * s, ph, sh, a.status)) { step_fail(sh, a.status, kDevTimeoutMma); ok = false; break; }
+                        if (k == 0 && kb == 0) stamp(a, img, 8, threadIdx.x);
                         tc_fence_after();
-                        const uint32_t st = smem_u32(region + s * ring_stage_bytes);
-                        const uint64_t a_hi = make_sw128_kmajor_desc(st);
-                        const uint64_t b_hi = make_sw128_kmajor_desc(st + Cfg::planes * a_bytes);
+                        const uint64_t a_hi = a_hi0 + off, b_hi = b_hi0 + off;
 #pragma unroll
                         for (uint32_t kk = 0; kk < kBlockK / kUmmaK; ++kk) {
                             const uint64_t adv = (kk * kUmmaK) >> 4;      // 32 bytes along K inside the swizzled row
@@ -338,19 +351,20 @@ train_steps_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
                             if (MODE == kModeU8) {
                                 mma(tmem_base, a_hi + adv, b_hi + adv, acc);
                             } else {
-                                const uint64_t a_lo = make_sw128_kmajor_desc(st + a_bytes);
-                                const uint64_t b_lo = make_sw128_kmajor_desc(st + Cfg::planes * a_bytes + pl.b_bytes);
+                                const uint64_t a_lo = a_hi + to_a_lo, b_lo = b_hi + to_b_lo;
                                 mma(tmem_base, a_hi + adv, b_hi + adv, acc);                         // hh
                                 mma(tmem_base + Cfg::max_n, a_lo + adv, b_lo + adv, acc);            // ll
                                 mma(tmem_base + 2 * Cfg::max_n, a_hi + adv, b_lo + adv, acc);        // cross
                                 mma(tmem_base + 2 * Cfg::max_n, a_lo + adv, b_hi + adv, 1u);
                             }
                         }
-                        commit(&sh.empty_bar[s]);        // frees the stage once these MMAs have read it
+                        commit(8 * s);                   // frees the stage once these MMAs have read it
+                        off += ring_stage_bytes >> 4;
+                        if (++s == stages) { s = 0; ph ^= 1; off = 0; }
                     }
                     if (!ok) break;
-                    commit(&sh.tmem_full);               // accumulators of this tile complete
-                    stamp(a, img, 9, 32);
+                    commit(smem_u32(&sh.tmem_full) - own0);   // accumulators of this tile complete
+                    stamp(a, img, 9, threadIdx.x);
                 }
             }
             __syncwarp();
