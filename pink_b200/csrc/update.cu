@@ -114,12 +114,12 @@ inline uint32_t div_magic(uint32_t d) { return d == 1 ? 0u : (uint32_t)((1ull <<
 // The kernel moves 12 bytes per pixel and computes next to nothing, so what counts is how many loads are in flight on
 // all SMs: with one block per neuron a map of 100 neurons left a third of the SMs idle and the others with 134 KB to
 // walk by eight warps; strips of 32 rows give every SM several blocks.  Per
-// image: 72.2 -> 15.4 us (100 neurons of 183 x 183), 12.1 -> 4.4 us (63 of 71 x 71), 7.7 -> 3.2 us (64 of 45 x 45).  A warp's load covers 4 rows x 8 columns: the base
+// image: 72.2 -> 12.6 us (100 neurons of 183 x 183), 12.1 -> 4.4 us (63 of 71 x 71), 7.7 -> 3.2 us (64 of 45 x 45).  A warp's load covers 4 rows x 8 columns: the base
 // rotation is read through the quarter-turn permutation, and a tile of that shape touches whole 16- or 32-byte
 // runs either way round (a row of 32 pixels would touch 32 lines for the odd quarter turns).
 // The strips of a neuron add their sums of squares into anorm, which worklist_kernel has zeroed.
 template <int MODE>
-__global__ void __launch_bounds__(kUpdThreads)
+__global__ void __launch_bounds__(kUpdThreads, 4)       // 64 registers: four blocks an SM (114: two, and a second wave, 15.4 us)
 update_kernel(const __grid_constant__ Geometry g, const __grid_constant__ UpdateArgs a, uint32_t strips)
 {
     __shared__ unsigned long long red[kUpdWarps];
