@@ -148,7 +148,7 @@ refine_f32_kernel(const float* __restrict__ A, const float* __restrict__ anorm, 
 // kernels give the same bits), but the block's warps share the scan of the estimates and form the exact sums of
 // different transforms at the same time.  A training step has one image's pairs only: as one warp per neuron they
 // filled a fifteenth of the GPU and every candidate's 2 x Kp floats were a chain of load latencies of its own.
-// 400 neurons x 720 transforms x 4096: 48.3 -> 13.9 us an image.  `dots` holds `splits` partial dot products of every pair
+// 400 neurons x 720 transforms x 4096: 48.3 -> 12.9 us an image.  `dots` holds `splits` partial dot products of every pair
 // ([splits][n][T], see launch_dots_tf32); adding them up costs splits - 1 roundings, fewer than the running sums
 // inside the tensor core lose by being shorter.  Shared memory: T estimates, then a list of T 16-bit indices.
 __global__ void __launch_bounds__(kRefineWarps * 32, 3)
@@ -167,8 +167,14 @@ refine_team_kernel(const float* __restrict__ A, const float* __restrict__ anorm,
     float ub = __int_as_float(0x7f800000);
     unsigned long long first = kKeyEmpty;
     for (uint32_t t = tid; t < T; t += kRefineWarps * 32) {
-        float dot = 0.0f;
-        for (uint32_t s = 0; s < splits; ++s) dot += dots[((size_t)s * n + nn) * T + t];
+        // every part's load in flight before the first is added (one after the other they are a chain of L2 latencies)
+        const float* part = dots + (size_t)nn * T + t;
+        const size_t step = (size_t)n * T;
+        float d[kMaxDotSplits], dot = 0.0f;
+#pragma unroll
+        for (uint32_t s = 0; s < kMaxDotSplits; ++s) d[s] = s < splits ? __ldg(part + s * step) : 0.0f;
+#pragma unroll
+        for (uint32_t s = 0; s < kMaxDotSplits; ++s) if (s < splits) dot += d[s];
         const float sum = __fadd_rn(na, bnorm[t]), v = fmaxf(sum - 2.0f * dot, 0.0f);
         est_s[t] = v;
         ub = fminf(ub, __fadd_rn(v, __fmul_rn(eps, sum)));
