@@ -215,8 +215,8 @@ struct pink_b200_ctx
     uint32_t* peer_rmax[kXchgMaxRanks] = {};
     uint64_t share_seq = 0;                                // batches handled so far (all ranks count alike)
     unsigned long long* d_stats = nullptr;   // [0] neurons with a non-zero factor, [1] neurons written back, summed over steps
-    // page-locked memory of the context: the device status word as check_status reads it, and (from kMailHead on) room
-    // for the results of small mapping calls, which the last kernel stores there itself
+    // page-locked memory, from the first small mapping call on (0.4 ms to get): the device status word as check_status reads
+    // it, and (from kMailHead on) the results of such calls, which the last kernel stores there itself
     uint8_t* h_mail = nullptr;
     uint64_t launches = 0;            // kernels launched by this context so far
     bool fuse_update = false;         // the update kernel finds the best matching unit and its work list itself
@@ -311,10 +311,10 @@ constexpr size_t kMailHead = 64, kMailResults = 64 * 1024;
 
 int check_status(pink_b200_ctx* c)
 {
-    CU_TRY(cudaMemcpyAsync(c->h_mail, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CU_TRY(cudaStreamSynchronize(c->stream));
     int st = 0;
-    std::memcpy(&st, c->h_mail, sizeof(int));
+    CU_TRY(cudaMemcpyAsync(c->h_mail ? static_cast<void*>(c->h_mail) : &st, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CU_TRY(cudaStreamSynchronize(c->stream));
+    if (c->h_mail) std::memcpy(&st, c->h_mail, sizeof(int));
     if (st != kDevOk) {
         // Sticky: the steps after the expired wait ran on whatever state it left, and with several ranks
         // the exchange counters no longer agree.  The context only answers get_som / destroy from here on.
@@ -994,7 +994,6 @@ int pink_b200_create(const pink_b200_config* cfg, pink_b200_ctx** out)
     CTX_TRY(cudaMemsetAsync(c->d_nitems, 0, 3 * sizeof(uint32_t), c->stream));
     CTX_TRY(cudaMalloc(&c->d_counts, N * sizeof(uint32_t)));
     CTX_TRY(cudaMemsetAsync(c->d_counts, 0, N * sizeof(uint32_t), c->stream));
-    CTX_TRY(cudaHostAlloc(&c->h_mail, kMailHead + kMailResults, cudaHostAllocDefault));
     CTX_TRY(cudaMalloc(&c->d_status, sizeof(int)));
     CTX_TRY(cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
 
@@ -1429,6 +1428,7 @@ int pink_b200_map(pink_b200_ctx* c, const float* host_images, uint64_t n, float*
     if (n <= B && n != 0 && total * 8 <= kMailResults) {
         // a small call is all latency: no second stream, and the last kernel stores the results in page-locked memory itself
         // (two pageable copies of a few hundred bytes took as long as the distance kernel; 100 neurons: 78 -> 55 us a call)
+        if (!c->h_mail) CU_TRY(cudaHostAlloc(&c->h_mail, kMailHead + kMailResults, cudaHostAllocDefault));
         float* hd = reinterpret_cast<float*>(c->h_mail + kMailHead);
         uint32_t* hr = reinterpret_cast<uint32_t*>(hd + total);
         CU_TRY(cudaStreamWaitEvent(c->stream, c->consumed[0], 0));
