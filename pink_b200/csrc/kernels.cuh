@@ -242,9 +242,9 @@ constexpr uint32_t kStepStampWords = 12;        // opt-in timeline words per ima
 // Control words of one launch; the host sets every byte to 0xFF before the launch.
 //   bmu_word[i]: minimum over all (neuron, transform tile) partial minima of image i of
 //                (code << s) | global neuron index, s = 32 (uint8) or 16 (uint16)
-//   bar:         arrival counter of the grid barriers (counts up from 0xFFFFFFFF, i.e. -1)
-//   failed:      cleared by a block whose wait expired; read together with bar in one 8-byte load
-struct StepCtrl { unsigned long long bmu_word[kStepBatchMax]; uint32_t bar; uint32_t failed; };
+//   bar:         the grid barriers' word, which starts at -1: low half arrivals, high half failed blocks (one 64-bit object:
+//                every access to it is 64 bits wide)
+struct StepCtrl { unsigned long long bmu_word[kStepBatchMax]; unsigned long long bar; };
 
 // Launch shape and shared-memory layout, fixed per context.
 struct StepPlan

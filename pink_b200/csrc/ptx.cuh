@@ -416,28 +416,16 @@ __device__ __forceinline__ unsigned long long global_timer_ns()
     return t;
 }
 
-__device__ __forceinline__ uint32_t ld_acquire_gpu_u32(const uint32_t* p)
-{
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ uint2 ld_acquire_gpu_u32x2(const void* p)      // p: 8-byte aligned
+__device__ __forceinline__ unsigned long long ld_acquire_gpu_u64(const unsigned long long* p)
 {
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+    return v;
 }
 
-__device__ __forceinline__ void red_release_gpu_add(uint32_t* p, uint32_t v)
+__device__ __forceinline__ void red_release_gpu_add(unsigned long long* p, unsigned long long v)
 {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ void st_relaxed_gpu_u32(uint32_t* p, uint32_t v)
-{
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
 }
 
 __device__ __forceinline__ int ld_relaxed_gpu_s32(const int* p)

@@ -38,7 +38,6 @@
 #include "tensormap.cuh"
 
 #include <algorithm>
-#include <cstddef>
 #include <type_traits>
 #include <vector>
 
@@ -61,6 +60,7 @@ constexpr int kMaxTasks = 2;                           // (row block, column) ta
 constexpr int kMaxUnits = 4;                           // operand groups of four elements per consumer thread and plane
 constexpr uint32_t kRegionBudget = 208 * 1024;         // shared memory the two phases use in turn
 constexpr unsigned long long kGridWaitNs = 2000000000ull;   // a grid barrier gives up after two seconds
+constexpr unsigned long long kBarArrived = 1ull, kBarFailed = 1ull << 32;   // what a block adds to the barrier word
 constexpr uint32_t kStampWords = kStepStampWords;
 
 template <int MODE> struct StepCfg;
@@ -140,23 +140,22 @@ __device__ __forceinline__ bool step_wait(uint64_t* bar, uint32_t parity, const 
 // Barrier over all blocks of the launch (all are resident: one per SM, cooperative launch).  `target`
 // is the number of arrivals since the launch began that completes it.
 // Two of these are on every image's critical path, so the thread that speaks for its block does as little as the memory model
-// asks for: one release (cumulative over what the block barrier ordered before it), then polls of one word pair that
-// hold the arrivals and the failure flag alike.  (Full fences on both sides and a separate read of the status word
-// took 1.8 us from the last arrival on; this form 1.2.)
+// asks for: one release (cumulative over what the block barrier ordered before it) that counts the arrival and, in the upper
+// half of the same word, a failure; then acquiring polls of that word.  All accesses are of the whole 64-bit word: a release
+// and an acquire of different widths on the same bytes would not synchronise.  (Full fences on both sides and a
+// separate read of the status word took 1.8 us from the last arrival on; one release and one poll 1.2.)
 __device__ __forceinline__ void grid_sync(const StepArgs& a, StepShared& sh, uint32_t target)
 {
-    static_assert(offsetof(StepCtrl, bar) % 8 == 0 && offsetof(StepCtrl, failed) == offsetof(StepCtrl, bar) + 4, "read as one word pair");
     __syncthreads();
     if (threadIdx.x == 0) {
         fence_proxy_async_all();          // this block's bulk stores to global memory are complete (waited for); order them too
-        if (step_aborted(sh)) st_relaxed_gpu_u32(&a.ctrl->failed, 0u);
-        red_release_gpu_add(&a.ctrl->bar, 1u);
+        red_release_gpu_add(&a.ctrl->bar, step_aborted(sh) ? kBarArrived + kBarFailed : kBarArrived);
         const unsigned long long t0 = global_timer_ns();
         uint32_t spins = 0;
         for (;;) {
-            const uint2 now = ld_acquire_gpu_u32x2(&a.ctrl->bar);
-            if (now.y == 0u) { *reinterpret_cast<volatile uint32_t*>(&sh.abort_flag) = 1u; break; }
-            if (now.x + 1u >= target) break;
+            const unsigned long long now = ld_acquire_gpu_u64(&a.ctrl->bar) + 1u;      // (the word starts at -1)
+            if (now >= kBarFailed) { *reinterpret_cast<volatile uint32_t*>(&sh.abort_flag) = 1u; break; }
+            if (now >= target) break;
             if ((++spins & 63u) == 0u && global_timer_ns() - t0 > kGridWaitNs) { step_fail(sh, a.status, kDevTimeoutGrid); break; }
         }
     }
