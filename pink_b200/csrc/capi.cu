@@ -15,6 +15,7 @@
 #include <dlfcn.h>
 #include <unistd.h>
 #include <nccl.h>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -215,9 +216,6 @@ struct pink_b200_ctx
     uint32_t* peer_rmax[kXchgMaxRanks] = {};
     uint64_t share_seq = 0;                                // batches handled so far (all ranks count alike)
     unsigned long long* d_stats = nullptr;   // [0] neurons with a non-zero factor, [1] neurons written back, summed over steps
-    // page-locked memory, from the first small mapping call on (0.4 ms to get): the device status word as check_status reads
-    // it, and (from kMailHead on) the results of such calls, which the last kernel stores there itself
-    uint8_t* h_mail = nullptr;
     uint64_t launches = 0;            // kernels launched by this context so far
     bool fuse_update = false;         // the update kernel finds the best matching unit and its work list itself
     // Whole batches of training steps in one persistent kernel (train_steps.cu) where the geometry allows it.
@@ -246,7 +244,9 @@ struct pink_b200_ctx
     bool failed = false;              // a device-side wait expired: the map may be inconsistent, training is refused
     uint32_t* d_counts = nullptr;
     uint32_t* d_bmu_log = nullptr; size_t bmu_log_cap = 0, bmu_log_n = 0;
+    // the device status word and, kMailHead bytes further on, room for the results of a small mapping call: one copy fetches both
     int* d_status = nullptr;
+    std::unique_ptr<uint8_t[]> h_mail;   // where that copy goes
     float* d_images[2] = { nullptr, nullptr }; size_t image_cap = 0;
     float* d_dist = nullptr; uint32_t* d_rot = nullptr; size_t out_imgs = 0;
     bool have_som = false, have_factors = false;
@@ -309,12 +309,15 @@ int ensure_image_staging(pink_b200_ctx* c, size_t imgs)
 
 constexpr size_t kMailHead = 64, kMailResults = 64 * 1024;
 
-int check_status(pink_b200_ctx* c)
+// Waits for the context's stream and looks at the device status word; `mail` (nullable) receives the word and what lies
+// behind it, `bytes` in all.
+int check_status(pink_b200_ctx* c, uint8_t* mail = nullptr, size_t bytes = 0)
 {
     int st = 0;
-    CU_TRY(cudaMemcpyAsync(c->h_mail ? static_cast<void*>(c->h_mail) : &st, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    if (mail) CU_TRY(cudaMemcpyAsync(mail, c->d_status, bytes, cudaMemcpyDeviceToHost, c->stream));
+    else CU_TRY(cudaMemcpyAsync(&st, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CU_TRY(cudaStreamSynchronize(c->stream));
-    if (c->h_mail) std::memcpy(&st, c->h_mail, sizeof(int));
+    if (mail) std::memcpy(&st, mail, sizeof(int));
     if (st != kDevOk) {
         // Sticky: the steps after the expired wait ran on whatever state it left, and with several ranks
         // the exchange counters no longer agree.  The context only answers get_som / destroy from here on.
@@ -994,8 +997,8 @@ int pink_b200_create(const pink_b200_config* cfg, pink_b200_ctx** out)
     CTX_TRY(cudaMemsetAsync(c->d_nitems, 0, 3 * sizeof(uint32_t), c->stream));
     CTX_TRY(cudaMalloc(&c->d_counts, N * sizeof(uint32_t)));
     CTX_TRY(cudaMemsetAsync(c->d_counts, 0, N * sizeof(uint32_t), c->stream));
-    CTX_TRY(cudaMalloc(&c->d_status, sizeof(int)));
-    CTX_TRY(cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
+    CTX_TRY(cudaMalloc(&c->d_status, kMailHead + kMailResults));
+    CTX_TRY(cudaMemsetAsync(c->d_status, 0, kMailHead, c->stream));
 
     // cos/sin of t * (float(2*pi)/R), t < R/4, evaluated on the host with the
     // reference's expressions (src/SelfOrganizingMapLib/generate_rotated_images.h:70,
@@ -1040,7 +1043,6 @@ int pink_b200_destroy(pink_b200_ctx* c)
     free_dev(c->d_circle); free_dev(c->d_owners); free_dev(c->d_ctrl); free_dev(c->d_stamps);
     for (cudaEvent_t e : c->prof_launch_events) cudaEventDestroy(e);
     free_dev(c->d_pairs); free_dev(c->d_counts); free_dev(c->d_bmu_log); free_dev(c->d_status);
-    if (c->h_mail) cudaFreeHost(c->h_mail);
     free_dev(c->d_images[0]); free_dev(c->d_images[1]); free_dev(c->d_dist); free_dev(c->d_rot);
     for (cudaEvent_t e : c->prof_events) cudaEventDestroy(e);
     for (cudaEvent_t e : c->prof_rot_events) cudaEventDestroy(e);
@@ -1426,20 +1428,20 @@ int pink_b200_map(pink_b200_ctx* c, const float* host_images, uint64_t n, float*
     }
     const size_t total = (size_t)n * c->count;
     if (n <= B && n != 0 && total * 8 <= kMailResults) {
-        // a small call is all latency: no second stream, and the last kernel stores the results in page-locked memory itself
-        // (two pageable copies of a few hundred bytes took as long as the distance kernel; 100 neurons: 78 -> 55 us a call)
-        if (!c->h_mail) CU_TRY(cudaHostAlloc(&c->h_mail, kMailHead + kMailResults, cudaHostAllocDefault));
-        float* hd = reinterpret_cast<float*>(c->h_mail + kMailHead);
-        uint32_t* hr = reinterpret_cast<uint32_t*>(hd + total);
+        // a small call is all latency: no second stream, and the results lie behind the status word, so that one copy
+        // fetches all three (a copy to pageable memory holds up the host for about 10 us, however few its bytes)
+        const size_t bytes = kMailHead + total * 8;
+        if (!c->h_mail) c->h_mail.reset(new uint8_t[kMailHead + kMailResults]);
+        float* dd = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(c->d_status) + kMailHead);
         CU_TRY(cudaStreamWaitEvent(c->stream, c->consumed[0], 0));
         CU_TRY(cudaMemcpyAsync(c->d_images[0], host_images, n * isz * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-        rc = map_chunk(c, c->d_images[0], (uint32_t)n, hd, hr);
+        rc = map_chunk(c, c->d_images[0], (uint32_t)n, dd, reinterpret_cast<uint32_t*>(dd + total));
         if (rc) return rc;
         CU_TRY(cudaEventRecord(c->consumed[0], c->stream));
-        rc = check_status(c);
+        rc = check_status(c, c->h_mail.get(), bytes);
         if (rc) return rc;
-        std::memcpy(host_dist, hd, total * sizeof(float));
-        std::memcpy(host_rot, hr, total * sizeof(uint32_t));
+        std::memcpy(host_dist, c->h_mail.get() + kMailHead, total * sizeof(float));
+        std::memcpy(host_rot, c->h_mail.get() + kMailHead + total * sizeof(float), total * sizeof(uint32_t));
         return PINK_B200_OK;
     }
     // Batches alternate between two staging/result buffers: the upload of batch k+1 and the download of batch k-1
