@@ -10,9 +10,14 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libpink_b200.so")
 SOURCES = ["capi.cu", "rotate.cu", "operands.cu", "distance_tc.cu", "distance_f32.cu", "filter_f32.cu", "update.cu", "train_steps.cu", "rotshare.cu", "group.cu", "mma_peak.cu", "host_tables.cpp"]
+# (object, source, macros): the rotation kernel's variants, a module each
+VARIANTS = [("rotate_%s_%s" % (mode[5:].lower(), kind[1:].lower()), "rotate.cu", ["-DPINK_ROTATE_MODE=" + mode, "-DPINK_ROTATE_KIND=" + kind])
+            for mode in ("kModeU8", "kModeU16", "kModeF32") for kind in ("kFast", "kCircle", "kLarge", "kPlanes")
+            if kind != "kPlanes" or mode == "kModeU8"]
 HEADERS = ["kernels.cuh", "ptx.cuh", "record.cuh", "quant.cuh", "tensormap.cuh", os.path.join("..", "..", "include", "pink_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC"]
+
 
 def _stale(target, deps):
     if not os.path.exists(target):
@@ -28,13 +33,13 @@ def build(force=False, verbose=False):
     os.makedirs(objdir, exist_ok=True)
     headers = [os.path.join(CSRC, h) for h in HEADERS]
     objs, procs = [], []
-    for src in SOURCES:
+    for name, src, macros in VARIANTS + [(os.path.splitext(src)[0], src, []) for src in SOURCES]:
         path = os.path.join(CSRC, src)
-        obj = os.path.join(objdir, os.path.splitext(src)[0] + ".o")
+        obj = os.path.join(objdir, name + ".o")
         objs.append(obj)
         if force or _stale(obj, [path] + headers):
             cmd = [nvcc] + NVCC_FLAGS + ["-Xcompiler", "-ffp-contract=off"] \
-                + (["-Xptxas", "-v"] if verbose else []) + ["-c", path, "-o", obj]
+                + (["-Xptxas", "-v"] if verbose else []) + macros + ["-c", path, "-o", obj]
             procs.append((cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     for cmd, p in procs:
         out, _ = p.communicate()

@@ -36,40 +36,15 @@
 
 namespace pinkb {
 
-namespace {
-
 constexpr uint32_t kRotMaxThreads = 1024;
 constexpr uint32_t kRotMaxGroup = 32;         // base rotations a block works through at most
 constexpr uint32_t kRotSmemBudget = 216 * 1024;
 constexpr uint32_t kRotHalfSm = 114 * 1024 - 1024 - 4096 - 256;   // dynamic shared memory of one of two blocks that share an SM
 
-// v / d for v * d < 2^32 with magic = floor(2^32 / d) + 1 (checked on the host).
-// magic == 0 encodes the divisor 1.
-__device__ __forceinline__ uint32_t fast_div(uint32_t v, uint32_t magic) { return magic ? __umulhi(v, magic) : v; }
-inline uint32_t div_magic(uint32_t d) { return d == 1 ? 0u : (uint32_t)((1ull << 32) / d) + 1; }
-
 template <int MODE> struct StageType;
 template <> struct StageType<kModeU8>  { using type = uint8_t; };
 template <> struct StageType<kModeU16> { using type = uint16_t; };
 template <> struct StageType<kModeF32> { using type = float; };
-
-template <int MODE>
-__device__ __forceinline__ typename StageType<MODE>::type to_stage(float v)
-{
-    if (MODE == kModeU8) return (typename StageType<MODE>::type)quant_u8(v);
-    if (MODE == kModeU16) return (typename StageType<MODE>::type)quant_u16(v);
-    return (typename StageType<MODE>::type)v;
-}
-
-// Shared-memory accesses by 32-bit shared-window address (one add per access instead of a generic pointer's arithmetic).
-__device__ __forceinline__ float lds_f32(uint32_t a) { float v; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); return v; }
-__device__ __forceinline__ float2 lds_f32x2(uint32_t a) { float2 v; asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a)); return v; }
-__device__ __forceinline__ uint32_t lds_u8(uint32_t a) { uint32_t v; asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
-__device__ __forceinline__ uint32_t lds_u16(uint32_t a) { uint32_t v; asm volatile("{ .reg .u16 t; ld.shared.u16 t, [%1]; cvt.u32.u16 %0, t; }" : "=r"(v) : "r"(a)); return v; }
-__device__ __forceinline__ uint4 lds_u32x4(uint32_t a) { uint4 v; asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a)); return v; }
-__device__ __forceinline__ void sts_f32(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" :: "r"(a), "f"(v) : "memory"); }
-__device__ __forceinline__ void sts_u8(uint32_t a, uint32_t v) { asm volatile("st.shared.u8 [%0], %1;" :: "r"(a), "r"(v) : "memory"); }
-__device__ __forceinline__ void sts_u16(uint32_t a, uint32_t v) { asm volatile("{ .reg .u16 t; cvt.u16.u32 t, %1; st.shared.u16 [%0], t; }" :: "r"(a), "r"(v) : "memory"); }
 
 // Launch shape and shared-memory layout.
 struct RotPlan
@@ -90,6 +65,40 @@ struct RotPlan
 // kPlanes (uint8, one channel) -- as kFast, but the pixels are scattered straight into the eight operand rows, which leave
 // shared memory as whole rows by bulk copies.
 enum : int { kFast = 0, kCircle = 1, kLarge = 2, kPlanes = 3 };
+
+// Launches rotate_kernel<MODE, ., KIND, .>; fills in rp.group and rp.groups.
+template <int MODE, int KIND>
+cudaError_t rotate_run(const Geometry& g, RotPlan& rp, bool inside, uint32_t n_img, size_t smem, const float* images, const float* cs, const float* sn,
+                       float* base_out, void* b0, void* b1, void* b2, void* bnorm, uint32_t* rmax, cudaStream_t st);
+
+// The file is compiled once for each (MODE, KIND) -- the kernels -- and once without the macros -- the choice between them.
+// The CUDA runtime loads a module whole when its first kernel is launched: with all 32 variants in one the first call of a
+// process took 2.4 ms longer than with a few.
+#ifdef PINK_ROTATE_MODE
+
+namespace {
+
+// v / d for v * d < 2^32 with magic = floor(2^32 / d) + 1 (checked on the host).
+// magic == 0 encodes the divisor 1.
+__device__ __forceinline__ uint32_t fast_div(uint32_t v, uint32_t magic) { return magic ? __umulhi(v, magic) : v; }
+
+template <int MODE>
+__device__ __forceinline__ typename StageType<MODE>::type to_stage(float v)
+{
+    if (MODE == kModeU8) return (typename StageType<MODE>::type)quant_u8(v);
+    if (MODE == kModeU16) return (typename StageType<MODE>::type)quant_u16(v);
+    return (typename StageType<MODE>::type)v;
+}
+
+// Shared-memory accesses by 32-bit shared-window address (one add per access instead of a generic pointer's arithmetic).
+__device__ __forceinline__ float lds_f32(uint32_t a) { float v; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); return v; }
+__device__ __forceinline__ float2 lds_f32x2(uint32_t a) { float2 v; asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a)); return v; }
+__device__ __forceinline__ uint32_t lds_u8(uint32_t a) { uint32_t v; asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ uint32_t lds_u16(uint32_t a) { uint32_t v; asm volatile("{ .reg .u16 t; ld.shared.u16 t, [%1]; cvt.u32.u16 %0, t; }" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ uint4 lds_u32x4(uint32_t a) { uint4 v; asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a)); return v; }
+__device__ __forceinline__ void sts_f32(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" :: "r"(a), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts_u8(uint32_t a, uint32_t v) { asm volatile("st.shared.u8 [%0], %1;" :: "r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts_u16(uint32_t a, uint32_t v) { asm volatile("{ .reg .u16 t; cvt.u16.u32 t, %1; st.shared.u16 [%0], t; }" :: "r"(a), "r"(v) : "memory"); }
 
 // INSIDE: the rotated window cannot leave the image at any angle -- half its diagonal, plus a margin far above the
 // rounding of the positions, lies within half the image -- so every source position s satisfies 0 <= s < id - 1:
@@ -499,18 +508,6 @@ rotate_kernel(const __grid_constant__ Geometry g, const __grid_constant__ RotPla
     if (KIND == kPlanes && !padded && threadIdx.x >= 32 && threadIdx.x < 32 + nv) bulk_wait_all();
 }
 
-// Row pitch (floats) of the staged image, at least `width`: the banks of an 8 x 4 tile of taps at any angle are the
-// points of the lattice {(dx, dy): dx * pitch + dy = 0 mod 32} away from one another; these residues keep the
-// lattice's shortest vector at 5.4 to 5.7 pixels (the densest possible packing has 6.1), so that a tile meets at most
-// two points of it and a read takes one to two passes.
-uint32_t bank_pitch(uint32_t width)
-{
-    for (uint32_t p = width;; ++p) {
-        const uint32_t r = p & 31u;
-        if (r == 6 || r == 7 || r == 9 || r == 23 || r == 25 || r == 26) return p;
-    }
-}
-
 template <int MODE, bool INSIDE, int KIND, int FLAGS>
 cudaError_t rotate_launch(const Geometry& g, RotPlan& rp, uint32_t n_img, size_t smem, const float* images, const float* cs, const float* sn,
                           float* base_out, void* b0, void* b1, void* b2, void* bnorm, uint32_t* rmax, cudaStream_t st)
@@ -541,6 +538,46 @@ cudaError_t rotate_launch(const Geometry& g, RotPlan& rp, uint32_t n_img, size_t
     }
     kernel<<<dim3(rp.groups, n_img), threads, smem, st>>>(g, rp, images, cs, sn, base_out, b0, b1, b2, bnorm, rmax);
     return cudaGetLastError();
+}
+
+} // namespace
+
+template <int MODE, int KIND>
+cudaError_t rotate_run(const Geometry& g, RotPlan& rp, bool inside, uint32_t n_img, size_t smem, const float* images, const float* cs, const float* sn,
+                       float* base_out, void* b0, void* b1, void* b2, void* bnorm, uint32_t* rmax, cudaStream_t st)
+{
+#define PINK_ROTATE(I, FLAGS) rotate_launch<MODE, I, KIND, FLAGS>(g, rp, n_img, smem, images, cs, sn, base_out, b0, b1, b2, bnorm, rmax, st)
+    if constexpr (KIND == kFast || KIND == kPlanes) {
+        // the common case -- a neuron that fits the image -- has its flags compiled in
+        if (!inside) return PINK_ROTATE(false, -1);
+        if (base_out) return rp.win == g.ed ? PINK_ROTATE(true, 3) : PINK_ROTATE(true, 1);
+        return rp.win == g.ed ? PINK_ROTATE(true, 2) : PINK_ROTATE(true, 0);
+    } else {
+        return inside ? PINK_ROTATE(true, -1) : PINK_ROTATE(false, -1);
+    }
+#undef PINK_ROTATE
+}
+
+template cudaError_t rotate_run<PINK_ROTATE_MODE, PINK_ROTATE_KIND>(const Geometry&, RotPlan&, bool, uint32_t, size_t, const float*, const float*,
+    const float*, float*, void*, void*, void*, void*, uint32_t*, cudaStream_t);
+
+#else
+
+namespace {
+
+inline uint32_t div_magic(uint32_t d) { return d == 1 ? 0u : (uint32_t)((1ull << 32) / d) + 1; }
+
+
+// Row pitch (floats) of the staged image, at least `width`: the banks of an 8 x 4 tile of taps at any angle are the
+// points of the lattice {(dx, dy): dx * pitch + dy = 0 mod 32} away from one another; these residues keep the
+// lattice's shortest vector at 5.4 to 5.7 pixels (the densest possible packing has 6.1), so that a tile meets at most
+// two points of it and a read takes one to two passes.
+uint32_t bank_pitch(uint32_t width)
+{
+    for (uint32_t p = width;; ++p) {
+        const uint32_t r = p & 31u;
+        if (r == 6 || r == 7 || r == 9 || r == 23 || r == 25 || r == 26) return p;
+    }
 }
 
 template <int MODE>
@@ -598,19 +635,12 @@ cudaError_t rotate_dispatch(const Geometry& g, const float* images, uint32_t n_i
     // -- unless it is what keeps a second block off the SM: then the threads store the pixels themselves
     if (smem <= kRotHalfSm && smem + plane > kRotHalfSm) rp.use_plane = 0;
     if (rp.use_plane) smem += plane;
-#define PINK_ROTATE(I, KIND, FLAGS) rotate_launch<MODE, I, KIND, FLAGS>(g, rp, n_img, smem, images, cs, sn, base_out, b0, b1, b2, bnorm, rmax, st)
-    // the common case -- a neuron that fits the image -- has its flags compiled in
-#define PINK_ROTATE_KIND(KIND)                                                                            \
-    if (!inside) return PINK_ROTATE(false, KIND, -1);                                                     \
-    if (base_out) return rp.win == g.ed ? PINK_ROTATE(true, KIND, 3) : PINK_ROTATE(true, KIND, 1);        \
-    return rp.win == g.ed ? PINK_ROTATE(true, KIND, 2) : PINK_ROTATE(true, KIND, 0);
+#define PINK_ROTATE(KIND) rotate_run<MODE, KIND>(g, rp, inside, n_img, smem, images, cs, sn, base_out, b0, b1, b2, bnorm, rmax, st)
     if (planes) {
-        if constexpr (MODE == kModeU8) { PINK_ROTATE_KIND(kPlanes) }
+        if constexpr (MODE == kModeU8) return PINK_ROTATE(kPlanes);
     }
-    if (!staged || !rp.use_region) return inside ? PINK_ROTATE(true, kLarge, -1) : PINK_ROTATE(false, kLarge, -1);
-    if (g.circle) return inside ? PINK_ROTATE(true, kCircle, -1) : PINK_ROTATE(false, kCircle, -1);
-    PINK_ROTATE_KIND(kFast)
-#undef PINK_ROTATE_KIND
+    if (!staged || !rp.use_region) return PINK_ROTATE(kLarge);
+    return g.circle ? PINK_ROTATE(kCircle) : PINK_ROTATE(kFast);
 #undef PINK_ROTATE
 }
 
@@ -625,5 +655,7 @@ cudaError_t launch_rotate(const Geometry& g, const float* images, uint32_t n_img
     // float: the planes are written only when both are given (b1 alone has no meaning in this mode)
     return rotate_dispatch<kModeF32>(g, images, n_img, cs, sn, base_out, base_plane, b0, b2 ? b1 : nullptr, b2, bnorm, rmax, st);
 }
+
+#endif // PINK_ROTATE_MODE
 
 } // namespace pinkb
