@@ -237,7 +237,8 @@ struct pink_b200_ctx
     // and of one mapping batch of transforms, the estimate matrix and the pass's counters
     float* d_af_hi = nullptr; float* d_af_lo = nullptr; float* d_af_norm = nullptr; bool af_valid = false;
     float* d_bf_hi = nullptr; float* d_bf_lo = nullptr; float* d_bf_norm = nullptr; float* d_est = nullptr; size_t filter_imgs = 0;
-    float* d_dots = nullptr;          // training: partial dot products of one image, [max_dot_splits][count][T]
+    DotPlan dot_plan{};               // training: how one image's dot products are split
+    float* d_dots = nullptr;          // training: their partial sums, [dot_plan.splits][count][T]
     unsigned long long* d_filter_stats = nullptr;     // {exact evaluations, bits of the largest estimate error seen}
     unsigned long long filter_pairs = 0;              // (neuron, transform) pairs estimated so far
     long long opt_exchange_timeout_ms = 20000;
@@ -431,11 +432,10 @@ int train_step(pink_b200_ctx* c, size_t slot_img, uint32_t* bmu_slot)
         fa.a0 = c->d_af_hi; fa.a1 = c->d_af_lo; fa.anorm = c->d_af_norm;
         fa.b0 = c->d_bf_hi; fa.b1 = c->d_bf_lo; fa.bnorm = c->d_bf_norm;
         fa.s_out = c->d_dots;
-        uint32_t splits = max_dot_splits(c);
-        e = launch_dots_tf32(g, fa, &splits, c->stream, &why);
+        e = launch_dots_tf32(g, fa, c->dot_plan, c->stream, &why);
         if (e == cudaSuccess) {
             why = "refine_team_kernel launch";
-            e = launch_refine_f32_dots(g, A, c->d_af_norm, c->count, B, c->d_bf_norm, c->d_dots, splits, filter_eps(g.K), c->d_keys,
+            e = launch_refine_f32_dots(g, A, c->d_af_norm, c->count, B, c->d_bf_norm, c->d_dots, c->dot_plan.splits, filter_eps(g.K), c->d_keys,
                                        c->d_filter_stats, c->stream);
         }
         c->filter_pairs += (unsigned long long)c->count * g.T;
@@ -855,7 +855,8 @@ int train_prepare(pink_b200_ctx* c, uint64_t n)
     if (uses_filter(c) && !c->use_steps) {
         int rcf = ensure_filter_buffers(c, c->filter_imgs ? c->filter_imgs : 1);
         if (rcf) return rcf;
-        if (!c->d_dots) CU_TRY(cudaMalloc(&c->d_dots, (size_t)max_dot_splits(c) * c->g.T * c->count * sizeof(float)));
+        if (!c->dot_plan.splits) c->dot_plan = plan_dots_tf32(c->g, c->count, !c->opt_mma_pairs, max_dot_splits(c));
+        if (!c->d_dots) CU_TRY(cudaMalloc(&c->d_dots, (size_t)c->dot_plan.splits * c->g.T * c->count * sizeof(float)));
     }
     if (!c->have_factors) return fail(PINK_B200_ESTATE, "pink_b200_set_update_factors must be called before training");
     if (c->cfg.world_size > 1 && !c->comm)

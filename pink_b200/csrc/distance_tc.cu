@@ -430,7 +430,7 @@ distance_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
 // ------------------------------------------------------------------ host side --
 
 template <int MODE, bool PAIR>
-cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st, const char** why, bool swap = false, uint32_t* splits = nullptr)
+cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st, const char** why, bool swap = false, const DotPlan* dots = nullptr)
 {
     using Cfg = TcCfg<MODE, PAIR>;
     using L = SmemLayout<MODE, PAIR>;
@@ -455,32 +455,9 @@ cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st,
         if (sms > 0 && rows * tiles < (uint64_t)sms)
             tiles = (uint32_t)std::max<uint64_t>(tiles, std::min<uint64_t>(most, (uint64_t)sms / rows));   // one wave
     }
-    auto tile_width = [&](uint32_t count) { return std::min<uint32_t>(Cfg::max_n, ((n_extent + count - 1) / count + 15) & ~15u); };
     const uint32_t slices = (uint32_t)((MODE == kModeTf32 ? 4ull : 1ull) * g.Kp / kBlockK);
-    uint32_t kb_split = slices;
-    if (splits) {
-        // One image's tiles alone leave most SMs idle or, narrow, make every SM pull the whole row tile (400 x 720 x 4096:
-        // 54 blocks of 5 MB, 40.6 us; now 16.6).  With K split too, the choice of column tiles and K ranges that
-        // moves the fewest bytes per SM: operand slices in, partial products out and in again.
-        const uint32_t max_splits = std::min(std::max(*splits, 1u), kMaxDotSplits);
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const uint64_t wave = sms > 0 ? sms : 148;
-        uint64_t best = ~0ull;
-        const uint32_t fewest = (n_extent + Cfg::max_n - 1) / Cfg::max_n, most = std::max<uint32_t>(fewest, n_extent / 32);
-        for (uint32_t count = fewest; count <= most; ++count) {
-            const uint32_t width = tile_width(count), columns = (n_extent + width - 1) / width, b = PAIR ? width / 2 : width;
-            for (uint32_t s = 1; s <= max_splits && (s == 1 || 2 * s <= slices); ++s) {
-                const uint64_t blocks = (uint64_t)m_tiles * columns * s, waves = (blocks + wave - 1) / wave;
-                const uint32_t len = (slices + s - 1) / s;
-                if ((s - 1) * len >= slices) continue;                // (the last range would be empty)
-                const uint64_t cost = waves * len * (kBlockM + b) * kBlockK * Cfg::planes + (uint64_t)s * a.n * g.T * 8 / wave;
-                if (cost < best) { best = cost; tiles = count; *splits = s; kb_split = len; }
-            }
-        }
-    }
-    const uint32_t n_tile = tile_width(tiles);
+    const uint32_t n_tile = dots ? dots->n_tile : std::min<uint32_t>(Cfg::max_n, ((n_extent + tiles - 1) / tiles + 15) & ~15u);
+    const uint32_t kb_split = dots ? dots->kb_split : slices, depth = dots ? dots->splits : a.n_img;      // depth: the grid's z
     const uint32_t n_tiles = (n_extent + n_tile - 1) / n_tile;
     const uint32_t b_box = PAIR ? n_tile / 2 : n_tile;         // column-side rows one CTA stages per K slice
 
@@ -520,7 +497,7 @@ cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st,
         cudaGetDevice(&dev2);
         if (dev2 != sm_dev2) { cudaDeviceGetAttribute(&sms2, cudaDevAttrMultiProcessorCount, dev2); sm_dev2 = dev2; }
         constexpr uint32_t half_sm = 113u * 1024u;                       // shared memory of one of two resident blocks
-        const uint64_t blocks = (uint64_t)m_tiles * n_tiles * a.n_img;
+        const uint64_t blocks = (uint64_t)m_tiles * n_tiles * depth;
         if (Cfg::cols <= 256 && sms2 > 0 && blocks > (uint64_t)sms2 && stages > 3
             && L::ring_off + 3 * stage_bytes + L::slack <= half_sm)
             stages = std::min(stages, (half_sm - L::ring_off - L::slack) / stage_bytes);
@@ -529,11 +506,11 @@ cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st,
     p.anorm = a.anorm; p.bnorm = a.bnorm; p.keys = a.keys; p.s_out = a.s_out; p.status = a.status;
     p.n = a.n; p.T = g.T; p.num_kb = num_kb; p.n_tile = n_tile; p.swap = swap ? 1u : 0u;
     p.stages = stages; p.b_bytes = b_bytes;
-    p.splits = splits ? *splits : 0u; p.kb_split = kb_split;
+    p.splits = dots ? dots->splits : 0u; p.kb_split = kb_split;
     p.tail_counter = a.tail ? a.tail_counter : nullptr;
     if (a.tail) p.tail = *a.tail;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(m_tiles, n_tiles, splits ? *splits : a.n_img);
+    cfg.gridDim = dim3(m_tiles, n_tiles, depth);
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = L::ring_off + stages * stage_bytes + L::slack;
     cfg.stream = st;
@@ -567,33 +544,33 @@ cudaError_t launch_distance_f32(const Geometry& g, const DistanceArgs& a, cudaSt
 
 // float32 filter pass: a0/a1 and b0/b1 are the TF32 word planes (high, low) of the operands, anorm/bnorm float
 // |.|^2, s_out [n_img][n][T] float receives the estimates; keys are not touched.  Needs Kp % 32 == 0.
-static cudaError_t estimate_tf32(const Geometry& g, const DistanceArgs& a, uint32_t* splits, cudaStream_t st, const char** why)
+static cudaError_t estimate_tf32(const Geometry& g, const DistanceArgs& a, bool swap, bool pair, const DotPlan* dots, cudaStream_t st, const char** why)
 {
     *why = "";
     if (a.n == 0 || a.n_img == 0) return cudaSuccess;
     if (g.Kp % 32 != 0 || !a.s_out) { *why = "launch_distance_tf32: operand stride or output"; return cudaErrorInvalidValue; }
-    // orientation: the one whose padded tile grid (rows to 128, or 256 for block pairs; columns to balanced tiles of
-    // at most 256, multiples of 16) computes fewer pairs that do not exist
-    auto padded = [](uint32_t m, uint32_t n) -> uint64_t {
-        const uint32_t mp = m > kBlockM ? (m + 2 * kBlockM - 1) / (2 * kBlockM) * (2 * kBlockM) : kBlockM;
-        const uint32_t tiles = (n + 255) / 256, nt = (((n + tiles - 1) / tiles) + 15) & ~15u;
-        return (uint64_t)mp * ((n + nt - 1) / nt) * nt;
-    };
-    const bool swap = padded(g.T, a.n) < padded(a.n, g.T);
-    const uint32_t m_extent = swap ? g.T : a.n;
-    if (m_extent > kBlockM && !a.single_cta) return launch_tc<kModeTf32, true>(g, a, st, why, swap, splits);
-    return launch_tc<kModeTf32, false>(g, a, st, why, swap, splits);
+    if (pair) return launch_tc<kModeTf32, true>(g, a, st, why, swap, dots);
+    return launch_tc<kModeTf32, false>(g, a, st, why, swap, dots);
 }
 
 cudaError_t launch_distance_tf32(const Geometry& g, const DistanceArgs& a, cudaStream_t st, const char** why)
 {
-    return estimate_tf32(g, a, nullptr, st, why);
+    const bool swap = estimate_swapped(a.n, g.T);
+    return estimate_tf32(g, a, swap, (swap ? g.T : a.n) > kBlockM && !a.single_cta, nullptr, st, why);
 }
 
-cudaError_t launch_dots_tf32(const Geometry& g, const DistanceArgs& a, uint32_t* splits, cudaStream_t st, const char** why)
+DotPlan plan_dots_tf32(const Geometry& g, uint32_t n, bool single_cta, uint32_t max_splits)
 {
-    if (a.n_img > 1) { *why = "launch_dots_tf32: one image"; return cudaErrorInvalidValue; }
-    return estimate_tf32(g, a, splits, st, why);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return plan_dots(n, g.T, g.Kp * 4 / kBlockK, single_cta, max_splits, sms > 0 ? (uint32_t)sms : 0u);
+}
+
+cudaError_t launch_dots_tf32(const Geometry& g, const DistanceArgs& a, const DotPlan& plan, cudaStream_t st, const char** why)
+{
+    if (a.n_img > 1 || plan.splits == 0) { *why = "launch_dots_tf32: one image, and a plan for it"; return cudaErrorInvalidValue; }
+    return estimate_tf32(g, a, plan.swap != 0, plan.pair != 0, &plan, st, why);
 }
 
 bool distance_has_tail(const Geometry& g) { return g.mode == kModeU8 || g.mode == kModeU16; }

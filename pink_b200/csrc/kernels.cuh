@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <functional>
 
+#include "dot_plan.hpp"
+
 struct pink_b200_config;
 
 namespace pinkb {
@@ -109,10 +111,10 @@ cudaError_t launch_distance(const Geometry& g, const DistanceArgs& a, cudaStream
 cudaError_t launch_split_tf32(const float* src, uint64_t rows, uint32_t Kp, float* hi, float* lo, float* norm, cudaStream_t st);
 cudaError_t launch_distance_tf32(const Geometry& g, const DistanceArgs& a, cudaStream_t st, const char** why);
 // For one image (training): launch_dots_tf32 leaves the dot products ah.bh + ah.bl + al.bh themselves, in partial sums over
-// ranges of K (a.s_out: [splits][n][T]; *splits: in the most that a.s_out holds, out the number used; norms are not read), and
+// ranges of K (a.s_out: [plan.splits][n][T]; norms are not read), as plan_dots_tf32 laid them out for this geometry, and
 // launch_refine_f32_dots adds them up, forms the estimates and goes on as launch_refine_f32.
-constexpr uint32_t kMaxDotSplits = 16;
-cudaError_t launch_dots_tf32(const Geometry& g, const DistanceArgs& a, uint32_t* splits, cudaStream_t st, const char** why);
+DotPlan plan_dots_tf32(const Geometry& g, uint32_t n, bool single_cta, uint32_t max_splits);
+cudaError_t launch_dots_tf32(const Geometry& g, const DistanceArgs& a, const DotPlan& plan, cudaStream_t st, const char** why);
 cudaError_t launch_refine_f32_dots(const Geometry& g, const float* A, const float* anorm, uint32_t n, const float* B, const float* bnorm,
                                    const float* dots, uint32_t splits, float eps, unsigned long long* keys,
                                    unsigned long long* cand_count, cudaStream_t st);
