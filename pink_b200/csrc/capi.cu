@@ -236,9 +236,9 @@ struct pink_b200_ctx
     // float32 mapping filter: TF32 word planes and float norms of the SOM operand (valid while the SOM is unchanged)
     // and of one mapping batch of transforms, the estimate matrix and the pass's counters
     float* d_af_hi = nullptr; float* d_af_lo = nullptr; float* d_af_norm = nullptr; bool af_valid = false;
-    float* d_bf_hi = nullptr; float* d_bf_lo = nullptr; float* d_bf_norm = nullptr; float* d_est = nullptr; size_t filter_imgs = 0;
+    float* d_bf_hi = nullptr; float* d_bf_lo = nullptr; float* d_bf_norm = nullptr; size_t filter_imgs = 0;
     DotPlan dot_plan{};               // training: how one image's dot products are split
-    float* d_dots = nullptr;          // training: their partial sums, [dot_plan.splits][count][T]
+    float* d_est = nullptr; size_t est_planes = 0;   // [est_planes][count][T]: a mapping batch's estimates, or one image's partial dot products
     unsigned long long* d_filter_stats = nullptr;     // {exact evaluations, bits of the largest estimate error seen}
     unsigned long long filter_pairs = 0;              // (neuron, transform) pairs estimated so far
     long long opt_exchange_timeout_ms = 20000;
@@ -340,7 +340,7 @@ bool uses_filter(const pink_b200_ctx* c)
 // Bound of the estimate's error relative to |a|^2 + |b|^2 (derived in filter_f32.cu): 3 * K / 16 * 2^-23 + 2^-17
 float filter_eps(uint32_t K) { return (float)(3.0 * K / 16.0 * 1.1920928955078125e-7 + 7.62939453125e-6); }
 
-// Ranges of K the estimate of one image may be split into: their partial products stay within 256 MB.
+// Ranges of K the estimate of one image may be split into: their partial products stay within 256 MB (or one plane, if that is more).
 uint32_t max_dot_splits(const pink_b200_ctx* c)
 {
     return (uint32_t)std::min<uint64_t>(kMaxDotSplits, std::max<uint64_t>(1, (1ull << 26) / ((uint64_t)c->count * c->g.T)));
@@ -359,7 +359,7 @@ int ensure_filter_buffers(pink_b200_ctx* c, size_t imgs)
         c->af_valid = false;
     }
     if (c->filter_imgs < imgs) {
-        free_dev(c->d_bf_hi); free_dev(c->d_bf_lo); free_dev(c->d_bf_norm); free_dev(c->d_est);
+        free_dev(c->d_bf_hi); free_dev(c->d_bf_lo); free_dev(c->d_bf_norm);
         const size_t rows = imgs * g.T;
         CU_TRY(cudaMalloc(&c->d_bf_hi, rows * g.Kp * sizeof(float)));
         CU_TRY(cudaMalloc(&c->d_bf_lo, rows * g.Kp * sizeof(float)));
@@ -367,9 +367,38 @@ int ensure_filter_buffers(pink_b200_ctx* c, size_t imgs)
         CU_TRY(cudaMemsetAsync(c->d_bf_hi, 0, rows * g.Kp * sizeof(float), c->stream));
         CU_TRY(cudaMemsetAsync(c->d_bf_lo, 0, rows * g.Kp * sizeof(float), c->stream));
         CU_TRY(cudaMalloc(&c->d_bf_norm, rows * sizeof(float)));
-        CU_TRY(cudaMalloc(&c->d_est, rows * c->count * sizeof(float)));
         c->filter_imgs = imgs;
     }
+    return PINK_B200_OK;
+}
+
+// At least `least` planes of the estimate's scratch, `want` where the device has the memory.  (Training and mapping use it in
+// turn, on one stream.)
+int ensure_estimate(pink_b200_ctx* c, size_t want, size_t least)
+{
+    if (c->est_planes >= want) return PINK_B200_OK;
+    least = std::max(least, std::max<size_t>(1, std::min(c->est_planes, want)));
+    free_dev(c->d_est);
+    c->est_planes = 0;
+    for (size_t planes = want;; planes = std::max(least, planes / 2)) {
+        const cudaError_t e = cudaMalloc(&c->d_est, planes * c->g.T * c->count * sizeof(float));
+        if (e == cudaSuccess) { c->est_planes = planes; return PINK_B200_OK; }
+        c->d_est = nullptr;
+        if (e != cudaErrorMemoryAllocation || planes == least)
+            return fail(PINK_B200_ECUDA, std::string("memory for the estimated distances: ") + cudaGetErrorString(e));
+        cudaGetLastError();              // fewer planes will do
+    }
+}
+
+// Lays out the split of one image's dot products for training, within the scratch that can be had: one plane at least.
+int ensure_dot_plan(pink_b200_ctx* c)
+{
+    if (c->dot_plan.splits && c->dot_plan.splits <= c->est_planes) return PINK_B200_OK;
+    DotPlan plan = plan_dots_tf32(c->g, c->count, !c->opt_mma_pairs, max_dot_splits(c));
+    const int rc = ensure_estimate(c, plan.splits, 1);
+    if (rc) return rc;
+    if (c->est_planes < plan.splits) plan = plan_dots_tf32(c->g, c->count, !c->opt_mma_pairs, (uint32_t)c->est_planes);
+    c->dot_plan = plan;
     return PINK_B200_OK;
 }
 
@@ -431,11 +460,11 @@ int train_step(pink_b200_ctx* c, size_t slot_img, uint32_t* bmu_slot)
         DistanceArgs fa = da;
         fa.a0 = c->d_af_hi; fa.a1 = c->d_af_lo; fa.anorm = c->d_af_norm;
         fa.b0 = c->d_bf_hi; fa.b1 = c->d_bf_lo; fa.bnorm = c->d_bf_norm;
-        fa.s_out = c->d_dots;
+        fa.s_out = c->d_est;
         e = launch_dots_tf32(g, fa, c->dot_plan, c->stream, &why);
         if (e == cudaSuccess) {
             why = "refine_team_kernel launch";
-            e = launch_refine_f32_dots(g, A, c->d_af_norm, c->count, B, c->d_bf_norm, c->d_dots, c->dot_plan.splits, filter_eps(g.K), c->d_keys,
+            e = launch_refine_f32_dots(g, A, c->d_af_norm, c->count, B, c->d_bf_norm, c->d_est, c->dot_plan.splits, filter_eps(g.K), c->d_keys,
                                        c->d_filter_stats, c->stream);
         }
         c->filter_pairs += (unsigned long long)c->count * g.T;
@@ -855,8 +884,6 @@ int train_prepare(pink_b200_ctx* c, uint64_t n)
     if (uses_filter(c) && !c->use_steps) {
         int rcf = ensure_filter_buffers(c, c->filter_imgs ? c->filter_imgs : 1);
         if (rcf) return rcf;
-        if (!c->dot_plan.splits) c->dot_plan = plan_dots_tf32(c->g, c->count, !c->opt_mma_pairs, max_dot_splits(c));
-        if (!c->d_dots) CU_TRY(cudaMalloc(&c->d_dots, (size_t)c->dot_plan.splits * c->g.T * c->count * sizeof(float)));
     }
     if (!c->have_factors) return fail(PINK_B200_ESTATE, "pink_b200_set_update_factors must be called before training");
     if (c->cfg.world_size > 1 && !c->comm)
@@ -869,6 +896,10 @@ int train_prepare(pink_b200_ctx* c, uint64_t n)
         free_dev(c->d_bmu_log);
         CU_TRY(cudaMalloc(&c->d_bmu_log, n * sizeof(uint32_t)));
         c->bmu_log_cap = n;
+    }
+    if (uses_filter(c) && !c->use_steps) {
+        rc = ensure_dot_plan(c);         // last: it makes do with the memory that is left
+        if (rc) return rc;
     }
     CU_TRY(cudaMemsetAsync(c->d_bmu_log, 0xFF, n * sizeof(uint32_t), c->stream));
     c->bmu_log_n = n;
@@ -1039,7 +1070,7 @@ int pink_b200_destroy(pink_b200_ctx* c)
     free_dev(c->d_cs); free_dev(c->d_sn); free_dev(c->d_factors); free_dev(c->d_coords); free_dev(c->d_lut); free_dev(c->d_base);
     free_dev(c->d_b0); free_dev(c->d_b1); free_dev(c->d_bnorm); free_dev(c->d_keys);
     free_dev(c->d_af_hi); free_dev(c->d_af_lo); free_dev(c->d_af_norm); free_dev(c->d_bf_hi); free_dev(c->d_bf_lo);
-    free_dev(c->d_bf_norm); free_dev(c->d_est); free_dev(c->d_dots); free_dev(c->d_filter_stats);
+    free_dev(c->d_bf_norm); free_dev(c->d_est); free_dev(c->d_filter_stats);
     free_dev(c->d_items); free_dev(c->d_nitems); free_dev(c->d_stats); free_dev(c->d_wrange); free_dev(c->d_rmax);
     free_dev(c->d_circle); free_dev(c->d_owners); free_dev(c->d_ctrl); free_dev(c->d_stamps);
     for (cudaEvent_t e : c->prof_launch_events) cudaEventDestroy(e);
@@ -1335,6 +1366,8 @@ static int map_chunk(pink_b200_ctx* c, const float* d_images, uint32_t m, float*
     const bool filter = uses_filter(c);
     if (filter) {
         int rc = ensure_filter_buffers(c, c->map_batch);
+        if (rc) return rc;
+        rc = ensure_estimate(c, c->map_batch, c->map_batch);
         if (rc) return rc;
         // the rotation kernel also writes the estimate's TF32 planes and norms of the transforms
         LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, g.Pc, c->d_b0, c->d_bf_hi,
