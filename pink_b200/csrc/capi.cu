@@ -32,11 +32,14 @@ int fail(int code, const std::string& msg)
     return code;
 }
 
+// (The runtime keeps a refused call's error until it is asked for it; the check behind a later launch would report it again.)
 #define CU_TRY(expr)                                                                              \
     do {                                                                                          \
         cudaError_t e_ = (expr);                                                                  \
-        if (e_ != cudaSuccess)                                                                    \
+        if (e_ != cudaSuccess) {                                                                  \
+            cudaGetLastError();                                                                   \
             return fail(PINK_B200_ECUDA, std::string(#expr) + ": " + cudaGetErrorString(e_));     \
+        }                                                                                         \
     } while (0)
 
 // ---- NCCL, resolved at run time so that single-GPU users need no NCCL at all ----
@@ -270,6 +273,7 @@ int ensure_transform_buffers(pink_b200_ctx* c, size_t imgs, size_t base_needed)
     const Geometry& g = c->g;
     if (c->b_imgs < imgs) {
         free_dev(c->d_b0); free_dev(c->d_b1); free_dev(c->d_bnorm);
+        c->b_imgs = 0;                   // (here and below: nothing is left if a larger buffer cannot be had)
         const size_t rows = imgs * g.T;
         CU_TRY(cudaMalloc(&c->d_b0, operand_plane_bytes(g, rows)));
         CU_TRY(cudaMemsetAsync(c->d_b0, 0, operand_plane_bytes(g, rows), c->stream));
@@ -282,12 +286,14 @@ int ensure_transform_buffers(pink_b200_ctx* c, size_t imgs, size_t base_needed)
     }
     if (c->base_imgs < base_needed) {
         free_dev(c->d_base);
+        c->base_imgs = 0;
         CU_TRY(cudaMalloc(&c->d_base, base_needed * (g.q ? g.q : 1) * (size_t)g.Pp * sizeof(float)));
         c->base_imgs = base_needed;
     }
     const size_t key_imgs_needed = imgs;
     if (c->key_imgs < key_imgs_needed) {
         free_dev(c->d_keys);
+        c->key_imgs = 0;
         CU_TRY(cudaMalloc(&c->d_keys, imgs * c->count * sizeof(unsigned long long)));
         LAUNCH_TRY(launch_fill_keys(c->d_keys, imgs * c->count, c->stream));
         c->launches += 1;
@@ -300,6 +306,7 @@ int ensure_transform_buffers(pink_b200_ctx* c, size_t imgs, size_t base_needed)
 int ensure_image_staging(pink_b200_ctx* c, size_t imgs)
 {
     if (c->image_cap >= imgs) return PINK_B200_OK;
+    c->image_cap = 0;
     for (int i = 0; i < 2; ++i) {
         free_dev(c->d_images[i]);
         CU_TRY(cudaMalloc(&c->d_images[i], imgs * c->image_size() * sizeof(float)));
@@ -349,7 +356,8 @@ uint32_t max_dot_splits(const pink_b200_ctx* c)
 int ensure_filter_buffers(pink_b200_ctx* c, size_t imgs)
 {
     const Geometry& g = c->g;
-    if (!c->d_af_hi) {
+    if (!c->d_filter_stats) {            // (the last of them)
+        free_dev(c->d_af_hi); free_dev(c->d_af_lo); free_dev(c->d_af_norm);
         const size_t elems = (size_t)c->count * g.Kp;
         CU_TRY(cudaMalloc(&c->d_af_hi, elems * sizeof(float)));
         CU_TRY(cudaMalloc(&c->d_af_lo, elems * sizeof(float)));
@@ -360,6 +368,7 @@ int ensure_filter_buffers(pink_b200_ctx* c, size_t imgs)
     }
     if (c->filter_imgs < imgs) {
         free_dev(c->d_bf_hi); free_dev(c->d_bf_lo); free_dev(c->d_bf_norm);
+        c->filter_imgs = 0;
         const size_t rows = imgs * g.T;
         CU_TRY(cudaMalloc(&c->d_bf_hi, rows * g.Kp * sizeof(float)));
         CU_TRY(cudaMalloc(&c->d_bf_lo, rows * g.Kp * sizeof(float)));
@@ -384,9 +393,9 @@ int ensure_estimate(pink_b200_ctx* c, size_t want, size_t least)
         const cudaError_t e = cudaMalloc(&c->d_est, planes * c->g.T * c->count * sizeof(float));
         if (e == cudaSuccess) { c->est_planes = planes; return PINK_B200_OK; }
         c->d_est = nullptr;
+        cudaGetLastError();
         if (e != cudaErrorMemoryAllocation || planes == least)
             return fail(PINK_B200_ECUDA, std::string("memory for the estimated distances: ") + cudaGetErrorString(e));
-        cudaGetLastError();              // fewer planes will do
     }
 }
 
@@ -894,6 +903,7 @@ int train_prepare(pink_b200_ctx* c, uint64_t n)
     c->use_steps = c->plan_ok && c->opt_step_kernel == 0 && c->d_owners && (c->cfg.world_size == 1 || c->xchg_on);
     if (c->bmu_log_cap < n) {
         free_dev(c->d_bmu_log);
+        c->bmu_log_cap = c->bmu_log_n = 0;
         CU_TRY(cudaMalloc(&c->d_bmu_log, n * sizeof(uint32_t)));
         c->bmu_log_cap = n;
     }
@@ -965,6 +975,7 @@ int pink_b200_create(const pink_b200_config* cfg, pink_b200_ctx** out)
     do {                                                                                          \
         cudaError_t e_ = (expr);                                                                  \
         if (e_ != cudaSuccess) {                                                                  \
+            cudaGetLastError();                                                                   \
             fail(PINK_B200_ECUDA, std::string(#expr) + ": " + cudaGetErrorString(e_));            \
             return bail(PINK_B200_ECUDA);                                                         \
         }                                                                                         \
@@ -1212,6 +1223,7 @@ int pink_b200_set_update_factors(pink_b200_ctx* c, const float* host_factors)
     CU_TRY(cudaSetDevice(c->cfg.device));
     CU_TRY(cudaStreamSynchronize(c->stream));
     const size_t N = c->cfg.n_neurons;
+    c->have_factors = false;
     free_dev(c->d_lut);
     if (!c->d_factors) CU_TRY(cudaMalloc(&c->d_factors, N * c->count * sizeof(float)));
     {
@@ -1254,6 +1266,7 @@ int pink_b200_set_update_lut(pink_b200_ctx* c, uint32_t som_layout, uint32_t dim
         return fail(PINK_B200_EINVAL, "unsupported SOM layout");
     CU_TRY(cudaSetDevice(c->cfg.device));
     CU_TRY(cudaStreamSynchronize(c->stream));
+    c->have_factors = false;
     free_dev(c->d_factors); free_dev(c->d_lut);
     if (!c->d_coords) CU_TRY(cudaMalloc(&c->d_coords, (size_t)N * sizeof(short4)));
     CU_TRY(cudaMalloc(&c->d_lut, (size_t)n_classes * sizeof(float)));
@@ -1456,6 +1469,7 @@ int pink_b200_map(pink_b200_ctx* c, const float* host_images, uint64_t n, float*
     if (rc) return rc;
     if (c->out_imgs < 2 * B) {
         free_dev(c->d_dist); free_dev(c->d_rot);
+        c->out_imgs = 0;
         CU_TRY(cudaMalloc(&c->d_dist, 2 * B * c->count * sizeof(float)));
         CU_TRY(cudaMalloc(&c->d_rot, 2 * B * c->count * sizeof(uint32_t)));
         c->out_imgs = 2 * B;

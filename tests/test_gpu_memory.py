@@ -1,5 +1,5 @@
-"""Device memory of float32 training: the scratch of the tensor-core estimate holds what the split of one image needs, and less
-where the device has no more."""
+"""Device memory: the scratch of float32 training's estimate holds what the split of one image needs, and less where the
+device has no more; a context outlives a call that the memory did not suffice for."""
 import numpy as np
 import pytest
 
@@ -71,3 +71,41 @@ def test_training_makes_do_with_less_scratch(cuda):
             cuda.cuda.empty_cache()
     assert got_bmus == bmus
     assert np.array_equal(got_som.view(np.uint32), som.view(np.uint32))
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+def test_context_outlives_a_refused_call(cuda, mode):
+    """Mapping needs larger buffers than training; where they cannot be had the call is refused, and the next calls -- training
+    first, whose smaller buffers went with the attempt -- find everything they need."""
+    import pink_b200.capi as capi
+    imgs = blob_images(4, IDIM, 1, seed=2).reshape(4, 1, IDIM, IDIM)
+    d_imgs = cuda.from_numpy(np.ascontiguousarray(imgs, dtype=np.float32)).cuda()
+    rng = np.random.default_rng(5)
+    som0 = rng.random((N, 1, ND, ND), dtype=np.float32)
+    F = O.update_factors(0, SIDE0, SIDE1, O.FUNC_GAUSSIAN, 1.1, 0.2)
+
+    def run(starve):
+        with Context(capi, make_config(capi, N, 1, IDIM, ND, ED, R, True, mode)) as ctx:
+            ctx.set_som(som0)
+            ctx.set_factors(F)
+            ctx.e.train_device(d_imgs.data_ptr(), 4)
+            ctx.e.synchronize()
+            if starve:
+                cuda.cuda.empty_cache()
+                free = cuda.cuda.mem_get_info()[0]
+                hog = cuda.empty(free - 24 * MB, dtype=cuda.uint8, device="cuda")
+                try:
+                    with pytest.raises(Exception, match="memory"):
+                        ctx.map(imgs)
+                finally:
+                    del hog
+                    cuda.cuda.empty_cache()
+            ctx.e.train_device(d_imgs.data_ptr(), 4)
+            bmus = list(ctx.e.bmu_log(4))
+            som = ctx.get_som(som0)
+            return bmus, som, ctx.map(imgs)
+
+    want, got = run(False), run(True)
+    assert want[0] == got[0]
+    for a, b in ((want[1], got[1]), (want[2][0], got[2][0]), (want[2][1], got[2][1])):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
