@@ -14,7 +14,7 @@ SOURCES = ["capi.cu", "rotate.cu", "operands.cu", "distance_tc.cu", "distance_f3
 VARIANTS = [("rotate_%s_%s" % (mode[5:].lower(), kind[1:].lower()), "rotate.cu", ["-DPINK_ROTATE_MODE=" + mode, "-DPINK_ROTATE_KIND=" + kind])
             for mode in ("kModeU8", "kModeU16", "kModeF32") for kind in ("kFast", "kCircle", "kLarge", "kPlanes")
             if kind != "kPlanes" or mode == "kModeU8"]
-HEADERS = ["kernels.cuh", "ptx.cuh", "record.cuh", "quant.cuh", "tensormap.cuh", "dot_plan.hpp", os.path.join("..", "..", "include", "pink_b200.h")]
+HEADERS = ["kernels.cuh", "ptx.cuh", "record.cuh", "quant.cuh", "tensormap.cuh", "dot_plan.hpp", "owners.hpp", os.path.join("..", "..", "include", "pink_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC"]
 

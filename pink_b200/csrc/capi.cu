@@ -6,6 +6,7 @@
 // the rotation sets (peer memory over NVLink; NCCL as fallback).
 #include "../../include/pink_b200.h"
 #include "kernels.cuh"
+#include "owners.hpp"
 
 #include <atomic>
 #include <cmath>
@@ -1240,8 +1241,10 @@ int pink_b200_set_update_factors(pink_b200_ctx* c, const float* host_factors)
     if (c->plan_ok) {
         // which block of the persistent kernel rewrites which neuron: spread every neighbourhood over the blocks
         std::vector<uint32_t> owners((size_t)c->plan.grid * c->plan.owned_per_block);
-        step_assign_owners([&](uint32_t i, uint32_t m) { return host_factors[(size_t)i * N + m]; }, c->first, c->stride,
-                           c->count, c->plan, owners.data());
+        assign_owners(c->count, c->plan.grid, c->plan.owned_per_block, owners.data(), [&](uint32_t i, auto add) {
+            const float* row = host_factors + (size_t)(c->first + i * c->stride) * N + c->first;
+            for (uint32_t m = 0; m < i; ++m) add(m, row[(size_t)m * c->stride]);
+        });
         CU_TRY(cudaMemcpyAsync(c->d_owners, owners.data(), owners.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
         CU_TRY(cudaStreamSynchronize(c->stream));
     }
@@ -1275,14 +1278,9 @@ int pink_b200_set_update_lut(pink_b200_ctx* c, uint32_t som_layout, uint32_t dim
     CU_TRY(cudaStreamSynchronize(c->stream));
     const bool hex = som_layout == PINK_B200_LAYOUT_HEXAGONAL;
     if (c->plan_ok) {
-        auto cls = [&](uint32_t i, uint32_t m) -> uint32_t {
-            const int dx = coords[4 * i] - coords[4 * m], dy = coords[4 * i + 1] - coords[4 * m + 1], dz = coords[4 * i + 2] - coords[4 * m + 2];
-            if (hex) return ((dx >= 0) == (dy >= 0)) ? (uint32_t)std::abs(dx + dy) : (uint32_t)std::max(std::abs(dx), std::abs(dy));
-            return ((uint32_t)std::abs(dz) * dim0 + (uint32_t)std::abs(dy)) * dim1 + (uint32_t)std::abs(dx);
-        };
         std::vector<uint32_t> owners((size_t)c->plan.grid * c->plan.owned_per_block);
-        step_assign_owners([&](uint32_t i, uint32_t m) { return host_lut[cls(i, m)]; }, c->first, c->stride, c->count, c->plan,
-                           owners.data());
+        assign_owners(c->count, c->plan.grid, c->plan.owned_per_block, owners.data(),
+                      NearNeurons(coords.data(), N, hex, dim0, dim1, host_lut, n_classes, c->first, c->stride));
         CU_TRY(cudaMemcpyAsync(c->d_owners, owners.data(), owners.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
         CU_TRY(cudaStreamSynchronize(c->stream));
     }

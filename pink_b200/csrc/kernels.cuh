@@ -6,7 +6,6 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
-#include <functional>
 
 #include "dot_plan.hpp"
 
@@ -287,11 +286,6 @@ struct StepArgs
 
 // Fills `plan` and returns true when the persistent kernel can run this geometry on the current device.
 bool step_plan(const Geometry& g, uint32_t n_local, uint32_t n_global, StepPlan* plan, const char** why_not);
-// Which block updates which neuron: owners[b * owned_per_block + j], balanced so that the neurons close to any
-// best matching unit (large update factors) are spread over different blocks.
-// closeness(i, m): update factor between global neurons i and m (any symmetric non-negative measure of nearness).
-void step_assign_owners(const std::function<float(uint32_t, uint32_t)>& closeness, uint32_t first, uint32_t stride,
-                        uint32_t count, const StepPlan& plan, uint32_t* owners);
 cudaError_t launch_train_steps(const Geometry& g, const StepPlan& plan, const StepArgs& a, cudaStream_t st, const char** why);
 
 // ---- mapping epilogue -------------------------------------------------------

@@ -26,7 +26,7 @@
 //                    operand rows of rewritten neurons and their sums of squares are re-emitted.
 //   grid barrier
 //
-// Ownership of neurons is static (a table built on the host, see step_assign_owners), so a block
+// Ownership of neurons is static (a table built on the host, see assign_owners), so a block
 // needs no compaction over all neurons to find its work.  The two phases use the same shared memory
 // in turn.  Every wait -- on an mbarrier, on the grid barrier, on another rank -- is bounded; when one
 // expires the block records a status code, raises its abort flag so that all later waits return at
@@ -859,32 +859,6 @@ bool step_plan(const Geometry& g, uint32_t n_local, uint32_t n_global, StepPlan*
     pl->owned_per_block = (n_local + blocks - 1) / blocks;
     if (pl->owned_per_block > kStepMaxOwned || pl->owned_per_block * g.C > kMaxEntries) { *why_not = "too many neurons per block"; return false; }
     return true;
-}
-
-// Greedy assignment in index order: a neuron goes to the block (with room left) whose neurons so far are
-// farthest from it, closeness measured by the update factors themselves -- the factor of (i, m) is large exactly when
-// i and m are rewritten together.  The neighbourhood of any best matching unit then spreads over the
-// blocks almost evenly (measured on a hexagonal map of 2791 neurons, sigma 3: at most 5-7 neurons of a
-// block among the ~700-1000 neurons an image rewrites, against 7-9 for a round-robin assignment).
-void step_assign_owners(const std::function<float(uint32_t, uint32_t)>& closeness, uint32_t first, uint32_t stride,
-                        uint32_t count, const StepPlan& pl, uint32_t* owners)
-{
-    const uint32_t G = pl.grid, J = pl.owned_per_block;
-    std::fill(owners, owners + (size_t)G * J, ~0u);
-    std::vector<uint32_t> color(count), load(G, 0);
-    std::vector<double> score(G);
-    for (uint32_t i = 0; i < count; ++i) {
-        std::fill(score.begin(), score.end(), 0.0);
-        const uint32_t gi = first + i * stride;
-        for (uint32_t m = 0; m < i; ++m) score[color[m]] += std::fabs((double)closeness(gi, first + m * stride));
-        uint32_t best = G;
-        for (uint32_t c = 0; c < G; ++c) {
-            if (load[c] >= J) continue;
-            if (best == G || score[c] < score[best] || (score[c] == score[best] && load[c] < load[best])) best = c;
-        }
-        color[i] = best;
-        owners[(size_t)best * J + load[best]++] = i;
-    }
 }
 
 cudaError_t launch_train_steps(const Geometry& g, const StepPlan& pl, const StepArgs& a, cudaStream_t st, const char** why)
