@@ -1718,7 +1718,8 @@ int pink_b200_op_rotate(const pink_b200_config* cfg, const float* dev_images, ui
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     rc = stage_tables(g, &d_cs, &d_sn, st);
     if (rc) return rc;
-    cudaError_t e = launch_rotate(g, dev_images, n_img, d_cs, d_sn, dev_base, g.nd * g.nd, dev_b0, dev_b1, dev_bnorm, st);
+    cudaError_t e = clear_operand_padding(g, (size_t)n_img * g.T, dev_b0, dev_b1, st);
+    if (e == cudaSuccess) e = launch_rotate(g, dev_images, n_img, d_cs, d_sn, dev_base, g.nd * g.nd, dev_b0, dev_b1, dev_bnorm, st);
     cudaStreamSynchronize(st);
     cudaFree(d_cs); cudaFree(d_sn);
     if (e != cudaSuccess) return fail(PINK_B200_ECUDA, std::string("rotate_kernel launch: ") + cudaGetErrorString(e));

@@ -75,6 +75,9 @@ struct BmuPair { unsigned long long code; unsigned long long neuron; };
 cudaError_t launch_rotate(const Geometry& g, const float* images, uint32_t n_img, const float* cs, const float* sn,
                    float* base_out, uint32_t base_plane, void* b0, void* b1, void* bnorm, cudaStream_t st, uint32_t* rmax = nullptr,
                    void* b2 = nullptr);
+// Zeroes the elements K .. Kp of `rows` operand rows (b1: uint16 only).  The kernel above writes K elements a row, and more or
+// less of the padding by its variant; a context's buffers are zeroed when they are made, a caller's are not.
+cudaError_t clear_operand_padding(const Geometry& g, size_t rows, void* b0, void* b1, cudaStream_t st);
 
 // ---- SOM operand ------------------------------------------------------------
 // som: [n][Pp] float.  a0/a1/anorm: as b0/b1/bnorm with one row per neuron.

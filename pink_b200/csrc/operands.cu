@@ -203,6 +203,7 @@ extern "C" int pink_b200_op_rotate_static(const pink_b200_config* cfg, const flo
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // The shared array still holds the previous call's table; the part this call uses is overwritten in full.
     e = cudaMemcpyAsync(scratch, table, 2 * nq * sizeof(float), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = clear_operand_padding(g, (size_t)n_img * g.T, dev_b0, dev_b1, st);
     if (e == cudaSuccess) e = launch_rotate(g, dev_images, n_img, scratch, scratch + nq, dev_base, g.nd * g.nd, dev_b0, dev_b1, dev_bnorm, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);      // `table` is reused by this thread's next call
     if (e != cudaSuccess) return report_error(PINK_B200_ECUDA, cudaGetErrorString(e));

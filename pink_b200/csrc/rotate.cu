@@ -656,6 +656,15 @@ cudaError_t launch_rotate(const Geometry& g, const float* images, uint32_t n_img
     return rotate_dispatch<kModeF32>(g, images, n_img, cs, sn, base_out, base_plane, b0, b2 ? b1 : nullptr, b2, bnorm, rmax, st);
 }
 
+cudaError_t clear_operand_padding(const Geometry& g, size_t rows, void* b0, void* b1, cudaStream_t st)
+{
+    const size_t esz = g.mode == kModeF32 ? 4 : 1, used = g.K * esz, pitch = g.Kp * esz;
+    if (rows == 0 || used == pitch) return cudaSuccess;
+    cudaError_t e = cudaMemset2DAsync(static_cast<uint8_t*>(b0) + used, pitch, 0, pitch - used, rows, st);
+    if (e == cudaSuccess && g.mode == kModeU16) e = cudaMemset2DAsync(static_cast<uint8_t*>(b1) + used, pitch, 0, pitch - used, rows, st);
+    return e;
+}
+
 #endif // PINK_ROTATE_MODE
 
 } // namespace pinkb

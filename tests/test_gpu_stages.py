@@ -109,6 +109,31 @@ def test_rotation_layouts(cuda, case, mode):
             assert not b0[rows, K:].any()
 
 
+@pytest.mark.parametrize("case", [(1, 20, 14, 11, True), (1, 40, 28, 19, True), (2, 40, 28, 11, True), (3, 24, 16, 7, False), (1, 300, 200, 125, True)])
+@pytest.mark.parametrize("mode", [2, 1, 0])
+@pytest.mark.parametrize("entry", ["pink_b200_op_rotate", "pink_b200_op_rotate_static"])
+def test_rotation_operand_padding(cuda, case, mode, entry):
+    """The rows that the single-stage entries write are zero beyond K whatever the caller's buffers held before."""
+    import pink_b200.capi as capi
+    C_, idim, nd, ed, flip = case
+    R, n_img = 8, 2
+    T = R * (2 if flip else 1)
+    K = C_ * ed * ed
+    Kp = capi.lib.pink_b200_operand_stride(K, mode)
+    cfg = make_config(capi, 1, C_, idim, nd, ed, R, flip, mode)
+    imgs = cuda.rand(n_img, C_, idim, idim, device="cuda")
+    base = cuda.empty(n_img, R // 4, C_, nd, nd, device="cuda")
+    dtype, fill = (cuda.float32, float("nan")) if mode == 0 else (cuda.uint8, 255)
+    b0 = cuda.full((n_img * T, Kp), fill, dtype=dtype, device="cuda")
+    b1 = cuda.full((n_img * T, Kp), fill, dtype=dtype, device="cuda") if mode == 1 else None
+    bnorm = cuda.empty(n_img * T, dtype=cuda.int64, device="cuda")
+    capi.check(getattr(capi.lib, entry)(C.byref(cfg), ptr(imgs), n_img, ptr(base), ptr(b0), ptr(b1), ptr(bnorm), None))
+    cuda.cuda.synchronize()
+    for b in (b0, b1):
+        if b is not None:
+            assert not b[:, K:].any() and K < Kp
+
+
 def _distance(torch, capi, a, b, mode, n_img=1, want_matrix=True):
     """a: (N, K), b: (n_img*T, K) in the mode's natural dtype."""
     N, K = a.shape
