@@ -265,10 +265,6 @@ struct pink_b200_ctx
 
 namespace {
 
-// A base rotation is staged in shared memory when it fits; only then can the
-// float copy in global memory be skipped (mapping never reads it back).
-bool base_fits_smem(const Geometry& g) { return (size_t)g.P * sizeof(float) <= 200 * 1024; }
-
 int ensure_transform_buffers(pink_b200_ctx* c, size_t imgs, size_t base_needed)
 {
     const Geometry& g = c->g;
@@ -1381,10 +1377,10 @@ static int map_chunk(pink_b200_ctx* c, const float* d_images, uint32_t m, float*
         rc = ensure_estimate(c, c->map_batch, c->map_batch);
         if (rc) return rc;
         // the rotation kernel also writes the estimate's TF32 planes and norms of the transforms
-        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, g.Pc, c->d_b0, c->d_bf_hi,
+        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, rotate_needs_base(g) ? c->d_base : nullptr, g.Pc, c->d_b0, c->d_bf_hi,
                                  c->d_bf_norm, c->stream, nullptr, c->d_bf_lo));
     } else {
-        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, base_fits_smem(g) ? nullptr : c->d_base, g.Pc, c->d_b0, c->d_b1, c->d_bnorm, c->stream));
+        LAUNCH_TRY(launch_rotate(g, d_images, m, c->d_cs, c->d_sn, rotate_needs_base(g) ? c->d_base : nullptr, g.Pc, c->d_b0, c->d_b1, c->d_bnorm, c->stream));
     }
     DistanceArgs da{};
     da.a0 = c->d_a0; da.a1 = c->d_a1; da.anorm = c->d_anorm; da.n = c->count;
@@ -1443,7 +1439,7 @@ int pink_b200_map_device(pink_b200_ctx* c, const float* dev_images, uint64_t n, 
     if (!c || ((!dev_images || !dev_dist || !dev_rot) && n)) return fail(PINK_B200_EINVAL, "null argument");
     if (!c->have_som) return fail(PINK_B200_ESTATE, "pink_b200_set_som must be called before mapping");
     CU_TRY(cudaSetDevice(c->cfg.device));
-    int rc = ensure_transform_buffers(c, c->map_batch, base_fits_smem(c->g) ? 0 : c->map_batch);
+    int rc = ensure_transform_buffers(c, c->map_batch, rotate_needs_base(c->g) ? c->map_batch : 0);
     if (rc) return rc;
     for (uint64_t done = 0; done < n;) {
         const uint32_t m = (uint32_t)(n - done < c->map_batch ? n - done : c->map_batch);
@@ -1461,7 +1457,7 @@ int pink_b200_map(pink_b200_ctx* c, const float* host_images, uint64_t n, float*
     if (!c->have_som) return fail(PINK_B200_ESTATE, "pink_b200_set_som must be called before mapping");
     CU_TRY(cudaSetDevice(c->cfg.device));
     const size_t B = c->map_batch, isz = c->image_size();
-    int rc = ensure_transform_buffers(c, B, base_fits_smem(c->g) ? 0 : B);
+    int rc = ensure_transform_buffers(c, B, rotate_needs_base(c->g) ? B : 0);
     if (rc) return rc;
     rc = ensure_image_staging(c, B > c->train_batch ? B : c->train_batch);
     if (rc) return rc;

@@ -64,7 +64,7 @@ struct BmuPair { unsigned long long code; unsigned long long neuron; };
 // ---- rotation set -----------------------------------------------------------
 // images: [n_img][C][id][id] float.  cs/sn: [q] cos/sin of t*2*pi/R (entry 0 unused).
 // base_out (nullable): [n_img][max(q,1)][C] float base rotations, base_plane (>= nd*nd) floats from one nd x nd plane to the next;
-// required when the distance region of a base rotation does not fit shared memory.
+// required where rotate_needs_base says so: the converted distance region (one channel) does not fit shared memory.
 // b0/b1: operand planes [n_img*T][Kp] (u8: b0; u16: b0 = high byte, b1 = low
 // byte; f32: b0 as float, and -- when b1 is given -- b1 / b2 the two TF32 word
 // planes of the mapping estimate: value with its low 13 mantissa bits cleared,
@@ -75,6 +75,7 @@ struct BmuPair { unsigned long long code; unsigned long long neuron; };
 cudaError_t launch_rotate(const Geometry& g, const float* images, uint32_t n_img, const float* cs, const float* sn,
                    float* base_out, uint32_t base_plane, void* b0, void* b1, void* bnorm, cudaStream_t st, uint32_t* rmax = nullptr,
                    void* b2 = nullptr);
+bool rotate_needs_base(const Geometry& g);
 // Zeroes the elements K .. Kp of `rows` operand rows (b1: uint16 only).  The kernel above writes K elements a row, and more or
 // less of the padding by its variant; a context's buffers are zeroed when they are made, a caller's are not.
 cudaError_t clear_operand_padding(const Geometry& g, size_t rows, void* b0, void* b1, cudaStream_t st);

@@ -580,6 +580,14 @@ uint32_t bank_pitch(uint32_t width)
     }
 }
 
+// Shared memory of the row and column terms of a window, and of the converted region (its rows one odd pitch apart).
+size_t table_bytes(uint32_t nx) { return (8 * (size_t)nx + 127) & ~size_t(127); }
+size_t staged_region_bytes(const Geometry& g)
+{
+    const uint32_t win = g.nd - 2 * g.off;
+    return ((size_t)win * (win | 1u) * (g.mode == kModeF32 ? 4 : g.mode == kModeU16 ? 2 : 1) + 127) & ~size_t(127);
+}
+
 template <int MODE>
 cudaError_t rotate_dispatch(const Geometry& g, const float* images, uint32_t n_img, const float* cs, const float* sn, float* base_out,
                             uint32_t base_plane, void* b0, void* b1, void* b2, void* bnorm, uint32_t* rmax, cudaStream_t st)
@@ -605,10 +613,10 @@ cudaError_t rotate_dispatch(const Geometry& g, const float* images, uint32_t n_i
     rp.r0 = lo > 0 ? (uint32_t)lo : 0u;
     rp.side = std::min<uint32_t>(g.id, hi < g.id ? (uint32_t)hi + 1 : g.id) - rp.r0;
     rp.pitch = bank_pitch(rp.side + 1);
-    const size_t region = (((size_t)rp.win * rp.sp * sizeof(typename StageType<MODE>::type)) + 127) & ~size_t(127);
+    const size_t region = staged_region_bytes(g);
     const size_t image = ((size_t)(rp.side + 1) * rp.pitch * 4 + 127) & ~size_t(127);
     const size_t plane = ((size_t)P1 * 4 + 127) & ~size_t(127);
-    size_t smem = (8 * (size_t)rp.nx + 127) & ~size_t(127);
+    size_t smem = table_bytes(rp.nx);
     if (smem > 64 * 1024) return cudaErrorInvalidValue;
     const size_t table = smem;
     // uint8, one channel: scatter into whole operand rows, in two sets (one filled while the other is copied out) as long
@@ -620,7 +628,7 @@ cudaError_t rotate_dispatch(const Geometry& g, const float* images, uint32_t n_i
     bool planes = MODE == kModeU8 && g.C == 1 && !g.circle && table + image + rows <= kRotSmemBudget;
     rp.row_bufs = planes && table + image + 2 * rows <= kRotHalfSm ? 2 : 1;
     rp.use_region = table + region <= kRotSmemBudget;
-    if (!rp.use_region && !base_out) return cudaErrorInvalidValue;
+    if (!rp.use_region && !base_out) return cudaErrorInvalidValue;      // (rotate_needs_base)
     if (planes) smem += rp.row_bufs * rows;
     else if (rp.use_region) smem += region;
     const bool staged = smem + image <= kRotSmemBudget;
@@ -655,6 +663,8 @@ cudaError_t launch_rotate(const Geometry& g, const float* images, uint32_t n_img
     // float: the planes are written only when both are given (b1 alone has no meaning in this mode)
     return rotate_dispatch<kModeF32>(g, images, n_img, cs, sn, base_out, base_plane, b0, b2 ? b1 : nullptr, b2, bnorm, rmax, st);
 }
+
+bool rotate_needs_base(const Geometry& g) { return table_bytes(g.nd - 2 * g.off) + staged_region_bytes(g) > kRotSmemBudget; }
 
 cudaError_t clear_operand_padding(const Geometry& g, size_t rows, void* b0, void* b1, cudaStream_t st)
 {

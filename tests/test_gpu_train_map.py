@@ -188,6 +188,39 @@ def test_float_step_equals_map(cuda, case):
             assert np.array_equal(got[bmu].view(np.uint32), (w - (w - near) * F[bmu, bmu]).astype(np.float32).view(np.uint32))
 
 
+@pytest.mark.parametrize("case", [
+    # C, id, nd, ed, mode: neurons of more than 200 KB whose distance region fits shared memory (one channel at a time), images that
+    # fit and ones that do not; the largest float region that fits and the smallest that does not
+    (1, 240, 227, 100, 2), (1, 330, 240, 101, 1), (3, 150, 132, 60, 2), (3, 150, 132, 61, 0), (1, 330, 240, 100, 0),
+    (1, 260, 250, 232, 0), (1, 260, 250, 233, 0),
+])
+def test_map_large_neurons(cuda, case):
+    """Mapping interpolates the region only, for neurons of any size: the oracle's distances, and no base rotations in memory."""
+    import pink_b200.capi as capi
+    C_, idim, nd, ed, mode = case
+    N, R = 3, 8
+    rng = np.random.default_rng(nd + ed)
+    som = rng.random((N, C_, nd, nd), dtype=np.float32)
+    imgs = rng.random((2, C_, idim, idim), dtype=np.float32)
+    with Context(capi, make_config(capi, N, C_, idim, nd, ed, R, True, mode)) as ctx:
+        ctx.set_som(som)
+        got_d, got_r = ctx.map(imgs)
+    for i in range(2):
+        want_d, want_r = O.map_image(som, imgs[i], ed, R, True, mode)
+        if mode == 0:
+            assert np.allclose(got_d[i], want_d, rtol=1e-5)
+        else:
+            assert np.array_equal(got_d[i], want_d)
+        assert np.array_equal(got_r[i], want_r)
+    # a rotation set large enough to see: 64 images x 90 base rotations would be 1.3 GB
+    if (nd, mode) == (240, 1):
+        with Context(capi, make_config(capi, N, C_, idim, nd, 20, 360, True, mode)) as ctx:
+            ctx.set_som(som)
+            before = cuda.cuda.mem_get_info()[0]
+            ctx.map(imgs)
+            assert before - cuda.cuda.mem_get_info()[0] < 900 << 20
+
+
 @pytest.mark.parametrize("case", TRAIN_CASES[:5])
 def test_train_float_mode(cuda, case):
     """float32: one teacher-forced step at a time; the SOM must match the oracle bit for bit whenever
