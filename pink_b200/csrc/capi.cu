@@ -761,7 +761,7 @@ int setup_peer_exchange(pink_b200_ctx* c)
     mine.share = group;
     if (mine.share) {
         const size_t imgs = std::max<size_t>(3 * kRotBatch, c->map_batch);
-        int rc0 = ensure_transform_buffers(c, imgs, 3 * kRotBatch);
+        int rc0 = ensure_transform_buffers(c, imgs, rotate_needs_base(c->g) ? imgs : 3 * kRotBatch);     // (base rotations as well)
         if (rc0) return rc0;
         CU_TRY(cudaMalloc(&c->d_rotflag, 3 * W * sizeof(unsigned long long)));
         CU_TRY(cudaMemsetAsync(c->d_rotflag, 0, 3 * W * sizeof(unsigned long long), c->stream));
