@@ -19,8 +19,9 @@
 //   addition may lose one unit in the last place of the running sum even if the unit truncates (observed: it
 //   does).  Even and odd K steps use separate accumulators, so an accumulator sees 3 * K / 16 additions of its own
 //   part of the sum: 3 * K / 16 * 2^-23 of the whole.
-// (Training splits K into up to 16 ranges of at least two slices, whose partial sums are added in float: an accumulator then
-// sees a range's share of those additions, and the fewer than 16 roundings of half a unit that join the ranges are less.)
+// (Training splits K into up to 16 ranges, all but the last of at least two 32-element slices, whose partial sums are added in
+// float: every further range takes six additions a slice off the other ranges' accumulators and costs one rounding of half
+// a unit, also where it has a single slice, so that the bound holds with room for any split.)
 // eps = 3 * K / 16 * 2^-23 + 2^-17.  The largest deviation seen among the evaluated pairs is recorded so that tests
 // can compare it with eps (C2: 0.3 of eps).
 #include "kernels.cuh"
@@ -144,9 +145,11 @@ refine_f32_kernel(const float* __restrict__ A, const float* __restrict__ anorm, 
     }
 }
 
-// One block per neuron of one image: the same selection and the same exact sums (lane by lane in the same order, so both
-// kernels give the same bits), but the block's warps share the scan of the estimates and form the exact sums of
-// different transforms at the same time.  A training step has one image's pairs only: as one warp per neuron they
+// One block per neuron of one image: the same minimum from the same exact sums (lane by lane in the same order, so both
+// kernels give the same bits).  The block's warps share the scan of the estimates and form the exact sums of different
+// transforms at the same time; for that they do without the first transform's exact distance as a further upper limit, so
+// that the transforms summed here contain those refine_f32_kernel sums, and now and then a few more.
+// A training step has one image's pairs only: as one warp per neuron they
 // filled a fifteenth of the GPU and every candidate's 2 x Kp floats were a chain of load latencies of its own.
 // 400 neurons x 720 transforms x 4096: 48.3 -> 12.9 us an image.  `dots` holds `splits` partial dot products of every pair
 // ([splits][n][T], see launch_dots_tf32); adding them up costs splits - 1 roundings, fewer than the running sums

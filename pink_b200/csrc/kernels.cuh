@@ -197,8 +197,8 @@ cudaError_t launch_bmu(const BmuArgs& a, uint32_t phase, cudaStream_t st);
 // ---- neighbourhood update ---------------------------------------------------
 struct UpdateArgs
 {
-    float* som;                       // [n][Pp]
-    const float* base;                // [max(q,1)][C][nd][nd] base rotations of the current image
+    float* som;                       // [n][Pp], Pp = C * Pc
+    const float* base;                // [max(q,1)][C][Pc] base rotations of the current image
     const UpdateItem* items; const uint32_t* n_items;   // work list from launch_bmu
     uint32_t n, first_item;           // local neurons (upper bound of the work list); list entry `items` points at
     void* a0; void* a1; void* anorm;  // SOM operand rows to refresh
@@ -273,7 +273,7 @@ struct StepArgs
     uint32_t b_row0;                  // row of the first image's transform 0 in that buffer
     unsigned long long* keys;         // [n], kKeyEmpty on entry and on exit
     // update phase
-    float* som;                       // [n][Pp]
+    float* som;                       // [n][Pp], Pp = C * Pc
     const float* base;                // base rotations of the first image; consecutive images follow
     uint2* wrange; const uint32_t* rmax;   // nullable together: value ranges (see cannot_change); rmax[i] for image i
     FactorSource factors;             // update factors of (best matching unit, neuron)

@@ -160,6 +160,38 @@ def test_odd_neuron_sides(cuda, case, mode):
             assert np.array_equal(gr[0], wr) and np.array_equal(gd[0], wd)
 
 
+@pytest.mark.parametrize("case", [(2, 50, 35, 35, 1), (3, 40, 27, 19, 0), (4, 30, 21, 14, 0), (1, 300, 260, 240, 0)])
+@pytest.mark.parametrize("step_kernel", [1, 2])
+def test_float_steps_of_odd_and_large_neurons(cuda, case, step_kernel):
+    """float32 on padded channel planes of several channels (and with a region of more than 200 KB), by the pipelined and by the
+    split update: the map goes in and comes out unchanged, and after each step every neuron is the oracle's update of
+    it, given the unit and the transforms that mapping the image before the step reports."""
+    import pink_b200.capi as capi
+    C_, idim, nd, ed, shape = case
+    N, R = 20, 8
+    rng = np.random.default_rng(nd * 10 + C_)
+    som0 = rng.random((N, C_, nd, nd), dtype=np.float32)
+    imgs = blob_images(3, idim, C_, seed=nd).reshape(3, C_, idim, idim)
+    F = O.update_factors(0, 5, 4, O.FUNC_GAUSSIAN, 1.1, 0.2)
+    cfg = make_config(capi, N, C_, idim, nd, ed, R, True, 0)
+    cfg.ed_shape = capi.CIRCULAR if shape else capi.QUADRATIC
+    with Context(capi, cfg, {"step_kernel": step_kernel}) as ctx:
+        ctx.set_som(som0)
+        som = ctx.get_som(som0)
+        assert np.array_equal(som.view(np.uint32), som0.view(np.uint32))
+        ctx.set_factors(F)
+        for img in imgs:
+            dist, best = ctx.map(img[None])
+            want_d, _ = O.map_image(som, img, ed, R, True, 0, shape=shape)
+            assert np.allclose(dist[0], want_d, rtol=1e-5)
+            bmu = int(ctx.train(img[None])[0])
+            assert bmu == int(dist[0].argmin())
+            near = O.rotation_set(img, nd, R, True)[best[0]]
+            want = (som - (som - near) * F[bmu][:, None, None, None]).astype(np.float32)
+            som = ctx.get_som(som0)
+            assert np.array_equal(som.view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("case", [
     # neurons, C, id, nd, ed, R, flip: one and several tiles on either side, both orientations of the estimate, one K slice
     # to hundreds (no split, uneven last ranges), transforms that are no multiple of four
