@@ -92,6 +92,7 @@ struct TcParams
     uint32_t n, T, num_kb, n_tile;
     uint32_t swap;              // kModeTf32 only: the transforms are the tile rows (M side), the neurons its columns
     uint32_t splits, kb_split;  // kModeTf32, one image: 0, or grid z = ranges of kb_split K slices whose raw dot products go to s_out[z]
+    uint32_t alloc_turns;       // PAIR: another pair may share this pair's SMs, so that they allocate tensor memory in turn
     uint32_t stages, b_bytes;   // ring depth; bytes of this CTA's transform rows per plane and stage (multiple of 1024)
     uint32_t* tail_counter;     // nullable: block arrival counter (zero between launches) that enables the tail below
     BmuArgs tail;               // the last block to finish reduces the shard's keys to its record and publishes it
@@ -100,6 +101,31 @@ struct TcParams
 __device__ __forceinline__ void report(int* status, int code)
 {
     if (status) atomicCAS(status, kDevOk, code);
+}
+
+// Turns of CTA pairs at allocating tensor memory, a word for every two SMs (the CTAs of a pair lie on SMs 2i and 2i + 1), shared
+// by all launches on the device.  The allocation of a pair takes the right to allocate on both SMs, one after the other; of
+// two pairs on the same SMs each could hold one of them and wait for the other's for good.  That takes two launches side by
+// side (several contexts, or streams): within one launch a pair starts long after the one before it on the same SMs.
+__device__ uint32_t g_alloc_turn[256];
+
+__device__ __forceinline__ uint32_t* alloc_turn_word()
+{
+    uint32_t sm;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    return &g_alloc_turn[(sm >> 1) & 255u];
+}
+
+// The holder runs on these SMs already and only has to allocate, so the wait ends; it is limited all the same.
+__device__ __forceinline__ bool take_alloc_turn(uint32_t* turn)
+{
+    if (atomicCAS(turn, 0u, 1u) == 0u) return true;
+    const unsigned long long t0 = global_timer_ns();
+    do {
+        __nanosleep(100);
+        if (atomicCAS(turn, 0u, 1u) == 0u) return true;
+    } while (global_timer_ns() - t0 < kMbarWaitNs);
+    return false;
 }
 
 template <int MODE, bool PAIR>
@@ -141,6 +167,15 @@ distance_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
         tma_prefetch_desc(&map_b0);
         if (Cfg::planes == 2) { tma_prefetch_desc(&map_a1); tma_prefetch_desc(&map_b1); }
     }
+    uint32_t* turn = nullptr;             // (one thread of the pair holds it)
+    if (PAIR && p.alloc_turns) {
+        if (pair_rank == 0 && threadIdx.x == 32) {
+            turn = alloc_turn_word();
+            if (!take_alloc_turn(turn)) { turn = nullptr; report(p.status, kDevTimeoutAlloc); }
+        }
+        __syncwarp();
+        cluster_sync();
+    }
     if (warp == 1) {
         if (PAIR) { tmem_alloc_pair(tmem_ptr_s, Cfg::cols); tmem_relinquish_pair(); }
         else { tmem_alloc(tmem_ptr_s, Cfg::cols); tmem_relinquish(); }
@@ -149,6 +184,7 @@ distance_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
     if (PAIR) cluster_sync();             // the peer's barriers are initialised before anything arrives on them
     else __syncthreads();
     tc_fence_after();
+    if (turn) atomicExch(turn, 0u);
     const uint32_t tmem_base = *tmem_ptr_s;
     // Everything above is independent of earlier kernels; the operands, norms and keys are not.
     griddep_launch();
@@ -394,6 +430,7 @@ distance_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
         }
     }
 
+    __syncwarp();                         // (one thread of the first two warps was at work; the barrier is for whole warps)
     tc_fence_before();
     if (PAIR) cluster_sync();             // neither CTA leaves while the other may still signal or read it
     else __syncthreads();
@@ -506,13 +543,17 @@ cudaError_t launch_tc(const Geometry& g, const DistanceArgs& a, cudaStream_t st,
     p.anorm = a.anorm; p.bnorm = a.bnorm; p.keys = a.keys; p.s_out = a.s_out; p.status = a.status;
     p.n = a.n; p.T = g.T; p.num_kb = num_kb; p.n_tile = n_tile; p.swap = swap ? 1u : 0u;
     p.stages = stages; p.b_bytes = b_bytes;
+    const size_t smem_bytes = L::ring_off + stages * stage_bytes + L::slack;
+    // beside a block of this size no other pair's fits an SM (227 KB; the smallest has two stages of 128 + 8 rows)
+    constexpr size_t smallest = L::ring_off + 2 * (L::a_bytes + 1024) + L::slack;
+    p.alloc_turns = PAIR && smem_bytes + smallest <= 227u * 1024u ? 1u : 0u;
     p.splits = dots ? dots->splits : 0u; p.kb_split = kb_split;
     p.tail_counter = a.tail ? a.tail_counter : nullptr;
     if (a.tail) p.tail = *a.tail;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(m_tiles, n_tiles, depth);
     cfg.blockDim = dim3(kThreads, 1, 1);
-    cfg.dynamicSmemBytes = L::ring_off + stages * stage_bytes + L::slack;
+    cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;

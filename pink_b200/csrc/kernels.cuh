@@ -18,7 +18,7 @@ enum : int { kModeF32 = 0, kModeU16 = 1, kModeU8 = 2 };
 constexpr int kModeTf32 = 3;      // internal: the tensor-core filter pass of float32 mapping (never a Geometry::mode)
 
 // Status codes a kernel may leave in the device status word.
-enum : int { kDevOk = 0, kDevTimeoutProducer = 1, kDevTimeoutMma = 2, kDevTimeoutEpilogue = 3,
+enum : int { kDevOk = 0, kDevTimeoutProducer = 1, kDevTimeoutMma = 2, kDevTimeoutEpilogue = 3, kDevTimeoutAlloc = 4,
              kDevTimeoutUpdateProducer = 11, kDevTimeoutUpdateConsumer = 12, kDevTimeoutExchange = 13, kDevTimeoutRotation = 14,
              kDevTimeoutGrid = 15 };
 

@@ -83,18 +83,36 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
 
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) { return mbar_try_wait(smem_u32(bar), parity); }
 
-// Each try_wait already blocks for a hardware-defined interval, so the limit
-// below corresponds to seconds, far beyond any legitimate wait in these kernels.
-constexpr uint32_t kSpinLimit = 1u << 22;
-
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
+// Nanoseconds of the device-wide timer: wall-clock limits of waits on other blocks or other GPUs.
+__device__ __forceinline__ unsigned long long global_timer_ns()
 {
-    for (uint32_t i = 0; i < kSpinLimit; ++i)
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Limits of a wait, far beyond any legitimate one in these kernels: a number of tries for the waits that look at a failure
+// flag between them, wall-clock time for the others (a try blocks for an interval that the hardware defines, so that a
+// number of tries alone says nothing about the time).
+constexpr uint32_t kSpinLimit = 1u << 22;
+constexpr unsigned long long kMbarWaitNs = 4000000000ull;
+
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned long long limit_ns = kMbarWaitNs)
+{
+    for (uint32_t i = 0; i < 64; ++i)
         if (mbar_try_wait(bar, parity)) return true;
+    const unsigned long long t0 = global_timer_ns();
+    do {
+        for (uint32_t i = 0; i < 64; ++i)
+            if (mbar_try_wait(bar, parity)) return true;
+    } while (global_timer_ns() - t0 < limit_ns);
     return false;
 }
 
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) { return mbar_wait(smem_u32(bar), parity); }
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned long long limit_ns = kMbarWaitNs)
+{
+    return mbar_wait(smem_u32(bar), parity, limit_ns);
+}
 
 // --------------------------------------------------------------------- TMA --
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map)
@@ -356,6 +374,8 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const CUtens
            "r"(x), "r"(y) : "memory");
 }
 
+// (Takes the right to allocate on the SMs of both CTAs.  Where another pair may run on the same two SMs, one pair at a time:
+// with the right of one SM each they would wait for one another.)
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols)
 {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -406,14 +426,6 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr)
 __device__ __forceinline__ void fence_proxy_async_all()
 {
     asm volatile("fence.proxy.async;" ::: "memory");
-}
-
-// Nanoseconds of the device-wide timer: wall-clock limits of waits on other blocks or other GPUs.
-__device__ __forceinline__ unsigned long long global_timer_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
 }
 
 __device__ __forceinline__ unsigned long long ld_acquire_gpu_u64(const unsigned long long* p)

@@ -204,6 +204,7 @@ train_steps_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
         tma_prefetch_desc(&map_b0);
         if (MODE == kModeU16) { tma_prefetch_desc(&map_a1); tma_prefetch_desc(&map_b1); }
     }
+    // (a block's registers fill its SM: no other pair allocates there at the same time)
     if (warp == 1) {
         if (PAIR) { tmem_alloc_pair(&sh.tmem_ptr, Cfg::cols); tmem_relinquish_pair(); }
         else { tmem_alloc(&sh.tmem_ptr, Cfg::cols); tmem_relinquish(); }

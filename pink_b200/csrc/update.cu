@@ -323,7 +323,7 @@ update_pipe_kernel(Geometry g, UpdateArgs a, PipeParams pp, BmuArgs b)
             for (uint32_t jx = 0; jx < m_fixed; ++jx) issue(jx);
         // the consumers publish the rest of the list and the factors
         uint32_t M = 0;
-        if (mbar_wait(&list_bar, 0)) M = m_s;
+        if (mbar_wait(&list_bar, 0, kMbarWaitNs + b.xchg_timeout_ns)) M = m_s;     // (they may wait for the other ranks' records)
         else if (pp.status) atomicCAS(pp.status, kDevOk, kDevTimeoutUpdateProducer);
         uint32_t n_live = 0, n_rewritten = 0;
         for (uint32_t jx = 0; jx < M; ++jx) {
